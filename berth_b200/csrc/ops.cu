@@ -139,7 +139,12 @@ __global__ void __launch_bounds__(256) k_add_f32(const float* a, const float* b,
 // order -- thread j folds the groups of four elements j, j + 128, ... with fmaf, the 128 partial sums are added by a
 // halving tree inside each warp and as (w0 + w1) + (w2 + w3) across the four warps -- and every other step is one
 // correctly rounded fp32 operation, so the rows equal the CPU checker's bit for bit.
-template <bool X_F16, bool W_BF16, bool RES_IN>
+//
+// Bound: the latency of a row's loads (one row per block; decode has few rows).  NC > 0: the thread's NC groups of the
+// row, and the weights beside them, are loaded at once and stay in registers between the two passes, so a row costs one
+// round of loads; a loop of dependent iterations paid the load latency ten times per pass at 5120 columns
+// (a two-layer decode step with four norms of one 5120-column row: 233.5 -> 211.1 us).  NC = 0: any dim, in a loop.
+template <bool X_F16, bool W_BF16, bool RES_IN, int NC>
 __global__ void __launch_bounds__(128) k_rms_norm(const void* __restrict__ x_, const uint16_t* __restrict__ w, __half* __restrict__ y,
                                                   float* __restrict__ residual, int dim, float eps, float bias, float scale)
 {
@@ -158,16 +163,47 @@ __global__ void __launch_bounds__(128) k_rms_norm(const void* __restrict__ x_, c
         }
         return v;
     };
+    auto res4 = [&](int c) { return reinterpret_cast<float4*>(residual + row * dim + 4 * c); };
     float s = 0.f;
-    for (int c = j; c < chunks; c += 128) {
-        float4 v = load4(c);
-        if constexpr (RES_IN) {
-            float4* rp = reinterpret_cast<float4*>(residual + row * dim + 4 * c);
-            const float4 r = *rp;
-            v = make_float4(__fadd_rn(r.x, v.x), __fadd_rn(r.y, v.y), __fadd_rn(r.z, v.z), __fadd_rn(r.w, v.w));
-            *rp = v;
-        }
+    auto fold = [&](const float4& v) {
         s = __fmaf_rn(v.x, v.x, s); s = __fmaf_rn(v.y, v.y, s); s = __fmaf_rn(v.z, v.z, s); s = __fmaf_rn(v.w, v.w, s);
+    };
+    auto add4 = [](const float4& r, const float4& v) {
+        return make_float4(__fadd_rn(r.x, v.x), __fadd_rn(r.y, v.y), __fadd_rn(r.z, v.z), __fadd_rn(r.w, v.w));
+    };
+    float4 held[NC > 0 ? NC : 1];
+    uint2 wheld[NC > 0 ? NC : 1];
+    if constexpr (NC > 0) {
+        float4 r[RES_IN ? NC : 1];
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+            const int c = j + 128 * i;
+            if (c < chunks) {
+                held[i] = load4(c);
+                if constexpr (RES_IN) r[i] = *res4(c);
+                wheld[i] = *reinterpret_cast<const uint2*>(w + 4 * c);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+            const int c = j + 128 * i;
+            if (c < chunks) {
+                if constexpr (RES_IN) {
+                    held[i] = add4(r[i], held[i]);
+                    *res4(c) = held[i];
+                }
+                fold(held[i]);
+            }
+        }
+    } else {
+        for (int c = j; c < chunks; c += 128) {
+            float4 v = load4(c);
+            if constexpr (RES_IN) {
+                v = add4(*res4(c), v);
+                *res4(c) = v;
+            }
+            fold(v);
+        }
     }
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, off));
@@ -176,11 +212,7 @@ __global__ void __launch_bounds__(128) k_rms_norm(const void* __restrict__ x_, c
     __syncthreads();
     const float total = __fadd_rn(__fadd_rn(ws[0], ws[1]), __fadd_rn(ws[2], ws[3]));
     const float rinv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, float(dim)), eps)));
-    for (int c = j; c < chunks; c += 128) {
-        float4 v;
-        if constexpr (RES_IN) v = *reinterpret_cast<const float4*>(residual + row * dim + 4 * c);   // this thread's own stores
-        else v = load4(c);
-        const uint2 wr = *reinterpret_cast<const uint2*>(w + 4 * c);
+    auto store4 = [&](int c, const float4& v, const uint2& wr) {
         float wf[4];
         if constexpr (W_BF16) {
             wf[0] = __uint_as_float(wr.x << 16); wf[1] = __uint_as_float(wr.x & 0xffff0000u);
@@ -198,6 +230,14 @@ __global__ void __launch_bounds__(128) k_rms_norm(const void* __restrict__ x_, c
         st.x = dq::pack_half2(o[0], o[1]);
         st.y = dq::pack_half2(o[2], o[3]);
         *reinterpret_cast<uint2*>(y + row * dim + 4 * c) = st;
+    };
+    if constexpr (NC > 0) {
+#pragma unroll
+        for (int i = 0; i < NC; ++i)
+            if (j + 128 * i < chunks) store4(j + 128 * i, held[i], wheld[i]);
+    } else {
+        for (int c = j; c < chunks; c += 128)   // (res_in: this thread's own stores)
+            store4(c, RES_IN ? *res4(c) : load4(c), *reinterpret_cast<const uint2*>(w + 4 * c));
     }
 }
 
@@ -214,8 +254,17 @@ void check_rms(const void* x, const void* w, const void* y, const void* r, int r
 template <bool X_F16, bool W_BF16, bool RES_IN>
 std::string launch_rms(const void* x, const void* w, void* y, void* r, int rows, int dim, float eps, float bias, float scale, cudaStream_t st)
 {
-    launch_pdl(k_rms_norm<X_F16, W_BF16, RES_IN>, dim3(rows), dim3(128), 0, st, "rms_norm launch", x, static_cast<const uint16_t*>(w),
-               static_cast<__half*>(y), static_cast<float*>(r), dim, eps, bias, scale);
+    // groups of four per thread held in registers: 4, 8, 12 or 16 (rows of up to 8192 columns), else the loop
+    auto go = [&](auto kern) {
+        launch_pdl(kern, dim3(rows), dim3(128), 0, st, "rms_norm launch", x, static_cast<const uint16_t*>(w), static_cast<__half*>(y),
+                   static_cast<float*>(r), dim, eps, bias, scale);
+    };
+    const int nc = (dim / 4 + 127) / 128;
+    if (nc <= 4) go(k_rms_norm<X_F16, W_BF16, RES_IN, 4>);
+    else if (nc <= 8) go(k_rms_norm<X_F16, W_BF16, RES_IN, 8>);
+    else if (nc <= 12) go(k_rms_norm<X_F16, W_BF16, RES_IN, 12>);
+    else if (nc <= 16) go(k_rms_norm<X_F16, W_BF16, RES_IN, 16>);
+    else go(k_rms_norm<X_F16, W_BF16, RES_IN, 0>);
     return std::string("k_rms_norm<") + (X_F16 ? "half" : "float") + "," + (W_BF16 ? "bfloat16" : "half") + (RES_IN ? ",res_in" : "") +
            "> block=128 grid=" + std::to_string(rows);
 }

@@ -73,74 +73,6 @@ struct LaneWords {
     static constexpr int value = (rmax + 7 * BITS + 16 + 31) / 32;
 };
 
-// Raw (little-endian uint16 pair) word -> stream order (first uint16 in the high half).
-__device__ __forceinline__ uint32_t stream_order(uint32_t raw) { return __byte_perm(raw, 0, 0x1032); }
-
-// Index of the first raw 32-bit word of the lane's span inside the tile, and the residual
-// left shift (a multiple of 8 below 32).
-template <int BITS>
-__device__ __forceinline__ void lane_span(int lane, int& word, int& shift)
-{
-    int bitpos = 8 * lane * BITS;
-    word = bitpos >> 5;
-    shift = bitpos & 31;
-}
-
-// Eight 16-bit states from the lane's stream-ordered words a0,a1,a2 (a2 ignored when the span
-// fits two words) already shifted so that the lane's first window starts at bit 31 of a0.
-template <int BITS>
-__device__ __forceinline__ void states_aligned(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t (&s)[8])
-{
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int p = j * BITS;
-        const int wi = p >> 5, sh = p & 31;
-        uint32_t hi = wi == 0 ? a0 : (wi == 1 ? a1 : a2);
-        uint32_t lo = wi == 0 ? a1 : (wi == 1 ? a2 : 0u);
-        s[j] = __funnelshift_l(lo, hi, sh) >> 16;
-    }
-}
-
-// Loads the lane's words from a tile (global or shared pointer to its 8*BITS raw words), with
-// the tail-biting wrap, and returns the eight states.
-template <int BITS>
-__device__ __forceinline__ void lane_states(const uint32_t* tile, int lane, uint32_t (&s)[8])
-{
-    constexpr int NW = 8 * BITS;
-    constexpr int NL = LaneWords<BITS>::value;
-    int w, r;
-    lane_span<BITS>(lane, w, r);
-    int w1 = w + 1; if (w1 >= NW) w1 -= NW;
-    uint32_t a0 = stream_order(tile[w]);
-    uint32_t a1 = stream_order(tile[w1]);
-    uint32_t a2 = 0;
-    if constexpr (NL > 2) {
-        int w2 = w1 + 1; if (w2 >= NW) w2 -= NW;
-        a2 = stream_order(tile[w2]);
-    }
-    if constexpr (BITS % 4 != 0) {
-        a0 = __funnelshift_l(a1, a0, r);
-        a1 = __funnelshift_l(a2, a1, r);
-        a2 = a2 << r;
-    }
-    states_aligned<BITS>(a0, a1, a2, s);
-}
-
-// Same from raw words already in registers (the order lane_states would load them in).
-template <int BITS>
-__device__ __forceinline__ void lane_states_regs(uint32_t r0, uint32_t r1, uint32_t r2, int lane, uint32_t (&s)[8])
-{
-    int w, r;
-    lane_span<BITS>(lane, w, r);
-    uint32_t a0 = stream_order(r0), a1 = stream_order(r1), a2 = stream_order(r2);
-    if constexpr (BITS % 4 != 0) {
-        a0 = __funnelshift_l(a1, a0, r);
-        a1 = __funnelshift_l(a2, a1, r);
-        a2 = a2 << r;
-    }
-    states_aligned<BITS>(a0, a1, a2, s);
-}
-
 // Half-word selection on the FMA-heavy pipe: dp2a.lo(a, b) = a.h0*b.byte0 + a.h1*b.byte1.
 __device__ __forceinline__ uint32_t lo16_heavy(uint32_t a)
 {
@@ -153,6 +85,66 @@ __device__ __forceinline__ uint32_t hi16_heavy(uint32_t a)
     uint32_t d;
     asm("dp2a.lo.u32.u32 %0, %1, 0x0100, 0;" : "=r"(d) : "r"(a));
     return d;
+}
+
+// Byte-permute selector that takes the lane's next four stream bytes, most significant first, from two neighbouring raw
+// words: a lane's span starts on a byte (lane*BITS bytes into the tile), so putting the words in stream order and
+// shifting them to the span's start is ONE permute per aligned word.  Nibble i = raw byte of stream byte rb+3-i,
+// which is (rb+3-i)^1 (the two bytes of a uint16 are swapped); constant over a kernel, so it is computed once.
+template <int BITS>
+__device__ __forceinline__ uint32_t align_selector(int lane)
+{
+    if constexpr (BITS % 4 == 0) return 0x1032u;
+    return uint32_t(0x2547325403251032ull >> (16 * ((lane * BITS) & 3))) & 0xffffu;
+}
+
+// Eight 16-bit states from the lane's words a0,a1,a2 (a2 ignored when the span fits two words), which hold its span
+// from its first bit on, most significant bit first: one shift brings a window to the low half of a word, one mask
+// cuts it out.  HEAVY = how many of the masks go to the FMA-heavy pipe instead of the ALU pipe, for balancing the two
+// integer pipes against the arithmetic of the codebook that follows.  Bound: the two pipes' issue rate.  Five instead of
+// eight ALU operations of set-up and the masks shared out: 21.1 / 19.1 / 19.1 -> 25.0 / 24.2 / 24.0 weights per clock and
+// SM at 3 / 5 / 6 bits on the integer path, 17.0 / 15.9 / 16.1 -> 18.2 / 18.0 / 17.9 on the fp16 path (MUL1, bare loops).
+template <int BITS, int HEAVY>
+__device__ __forceinline__ void states_aligned(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t (&s)[8])
+{
+    int heavy = HEAVY;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int p = j * BITS;
+        const int wi = p >> 5, sh = p & 31;
+        const uint32_t hi = wi == 0 ? a0 : (wi == 1 ? a1 : a2);
+        const uint32_t lo = wi == 0 ? a1 : (wi == 1 ? a2 : 0u);
+        if (sh == 8) {
+            s[j] = __byte_perm(hi, 0u, 0x4421);
+        } else if (sh == 0) {
+            s[j] = heavy > 0 ? hi16_heavy(hi) : hi >> 16;
+            --heavy;
+        } else {
+            const uint32_t w = sh <= 16 ? hi >> (16 - sh) : __funnelshift_l(lo, hi, sh - 16);   // window in the low half
+            s[j] = heavy > 0 ? lo16_heavy(w) : w & 0xffffu;
+            --heavy;
+        }
+    }
+}
+
+// Loads the lane's words from a tile (global or shared pointer to its 8*BITS raw words), with
+// the tail-biting wrap, and returns the eight states.
+template <int BITS, int HEAVY = 0>
+__device__ __forceinline__ void lane_states(const uint32_t* tile, int lane, uint32_t (&s)[8])
+{
+    constexpr int NW = 8 * BITS;
+    constexpr int NL = LaneWords<BITS>::value;
+    const int w = (lane * BITS) >> 2;
+    int w1 = w + 1; if (w1 >= NW) w1 -= NW;
+    const uint32_t sel = align_selector<BITS>(lane);
+    const uint32_t r0 = tile[w], r1 = tile[w1];
+    uint32_t r2 = r1;
+    if constexpr (NL > 2) {
+        int w2 = w1 + 1; if (w2 >= NW) w2 -= NW;
+        r2 = tile[w2];
+    }
+    // (the bytes an aligned word takes from past the last raw word lie behind the lane's last window)
+    states_aligned<BITS, HEAVY>(__byte_perm(r0, r1, sel), __byte_perm(r1, r2, sel), 7 * BITS + 16 > 64 ? __byte_perm(r2, r2, sel) : 0u, s);
 }
 
 // 4-bit tiles: eight 16-bit windows from the lane's raw word r0 and the next lane's r1
@@ -219,7 +211,7 @@ __device__ __forceinline__ void tile_states(const uint32_t* tile, int lane, int 
 {
     // the codebooks whose arithmetic leans on the ALU pipe take their half-word selections on the FMA-heavy pipe
     if constexpr (BITS == 4) states_4bit<(CB != 2) ? 6 : 0>(tile[lane], tile[lane1], s);
-    else lane_states<BITS>(tile, lane, s);
+    else lane_states<BITS, (CB != 2) ? 8 : 2>(tile, lane, s);
 }
 
 // Duplicated activation pairs for the lo/hi-as-k-slots scheme: from b0 = (x[2q], x[2q+1]) and
@@ -307,7 +299,7 @@ template <int BITS>
 __device__ __forceinline__ void tile_states_i8(const uint32_t* tile, int lane, int lane1, uint32_t (&s)[8])
 {
     if constexpr (BITS == 4) states_4bit<BERTH_I8_HEAVY>(tile[lane], tile[lane1], s);
-    else lane_states<BITS>(tile, lane, s);
+    else lane_states<BITS, 5>(tile, lane, s);
 }
 
 // One 16x16 tile against NG groups of four tokens.  Lane 4g+q holds the weights of output columns

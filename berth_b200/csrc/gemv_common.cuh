@@ -186,12 +186,13 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint
 // One 128-block of one activation row, whole warp: fp16(H128(x * suh) / sqrt(128)); the lane gets
 // elements 4*lane .. 4*lane+3 packed as two half pairs.  SUM: `sx` = sum of the 128 rounded values
 // (every lane), which the MUL1 epilogue needs.
+// `exact` (may be null): the four values before that rounding.
 template <bool SUM>
-__device__ __forceinline__ uint2 rotate_bits(uint2 xr, uint2 sr, int lane, float& sx);
+__device__ __forceinline__ uint2 rotate_bits(uint2 xr, uint2 sr, int lane, float& sx, float* exact = nullptr);
 
 template <bool SUM>
 __device__ __forceinline__ uint2 rotate_block(const __half* __restrict__ xrow, const __half* __restrict__ suh, int kb, int lane, float& sx,
-                                              const __half* __restrict__ urow = nullptr, float act_limit = 0.f)
+                                              const __half* __restrict__ urow = nullptr, float act_limit = 0.f, float* exact = nullptr)
 {
     const int kcol = kb * 128 + lane * 4;
     uint2 xr = *reinterpret_cast<const uint2*>(xrow + kcol);
@@ -206,12 +207,12 @@ __device__ __forceinline__ uint2 rotate_block(const __half* __restrict__ xrow, c
         xr.x = dq::pack_half2(o[0], o[1]);
         xr.y = dq::pack_half2(o[2], o[3]);
     }
-    return rotate_bits<SUM>(xr, sr, lane, sx);
+    return rotate_bits<SUM>(xr, sr, lane, sx, exact);
 }
 
 // The same from the lane's four input values and four scales, already loaded.
 template <bool SUM>
-__device__ __forceinline__ uint2 rotate_bits(uint2 xr, uint2 sr, int lane, float& sx)
+__device__ __forceinline__ uint2 rotate_bits(uint2 xr, uint2 sr, int lane, float& sx, float* exact)
 {
     __half2 x0 = *reinterpret_cast<__half2*>(&xr.x), x1 = *reinterpret_cast<__half2*>(&xr.y);
     __half2 s0 = *reinterpret_cast<__half2*>(&sr.x), s1 = *reinterpret_cast<__half2*>(&sr.y);
@@ -223,7 +224,11 @@ __device__ __forceinline__ uint2 rotate_bits(uint2 xr, uint2 sr, int lane, float
     dq::had128_warp(v, lane);
     __half h[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) h[i] = __float2half_rn(__fmul_rn(v[i], kRScale));
+    for (int i = 0; i < 4; ++i) {
+        const float r = __fmul_rn(v[i], kRScale);
+        if (exact) exact[i] = r;
+        h[i] = __float2half_rn(r);
+    }
     uint2 o;
     o.x = dq::pack_half2(h[0], h[1]);
     o.y = dq::pack_half2(h[2], h[3]);

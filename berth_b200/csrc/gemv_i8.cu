@@ -15,10 +15,12 @@
 // enter as 16-bit block fixed point: per (row, 128 rotated inputs) one fp32 scale = max|a| / 32512 and
 // v = rint(a / scale), split into two signed 8-bit limbs v = 256 hi + lo.  The limbs of a row are two
 // of the N columns of the MMA; the s32 accumulation is exact and is folded into an fp32 accumulator
-// once per 128 inputs: acc += scale * (256 hi_sum + lo_sum).  The constant term uses the same
+// once per 128 inputs: acc += 2 scale * (128 hi_sum + lo_sum / 2).  The constant term uses the same
 // quantised values (block sums = scale * sum v), so the result is exactly the product with the
-// quantised activations up to fp32 rounding; the quantisation step is 2^-15 of the block maximum,
-// finer than the fp16 rounding of the rotated activations that every path of this library shares.
+// quantised activations up to fp32 rounding.  The fp32 rotated values are quantised, not their fp16
+// roundings (which the caller's buffer receives): the step is 2^-15 of the block maximum, a rounding error of
+// 2.6e-5 of the block's root mean square where fp16 rounding makes 2e-4 (a linear's relative error against
+// 64 bits: 2.95e-4 with the fp16 roundings quantised, 2.1e-4 now; the rest is the codebook's own fp16 rounding).
 //
 // Work decomposition, TMA ring, split-K slabs and the finishing kernel are those of gemv.cu: units of
 // 128 inputs x BU*128 outputs in band-group-major order, CTA c takes a contiguous range.  Inside a CTA
@@ -172,7 +174,7 @@ __device__ __forceinline__ bool elect_one()
 }
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); }
 
-// The lane's four rotated fp16 values of one 128-block (lane = 4 consecutive inputs) -> block fixed point.
+// The lane's four rotated values of one 128-block, not yet rounded to fp16, (lane = 4 consecutive inputs) -> block fixed point.
 // Writes the two limbs of each value, replicated over the four bytes of a 32-bit word (the four u8 k-slots of a
 // weight's product), at their place in the block's limb tile: `tile_row` = tile + (row / 4) * 256 +
 // 2 * (row % 4) * 16, k-step stride `chunk_stride`, core-matrix stride `lbo` (256 * row groups and 128 in a ring
@@ -180,10 +182,8 @@ __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n
 // [core matrix 2][limb row 8][16 bytes], limb row = 2 * (row % 4) + (0 high, 1 low); k-step c of a k-tile row
 // holds, in this order, the inputs 2c (c < 4) and 2(c-4)+1 of its eight.  Returns the block's scale
 // (max|a| / 32512) and, in every lane, the sum of the block's 128 integers.
-__device__ __forceinline__ float quantise_block(uint2 o, int lane, unsigned char* tile_row, int chunk_stride, int lbo, int& isum)
+__device__ __forceinline__ float quantise_block(const float (&hv)[4], int lane, unsigned char* tile_row, int chunk_stride, int lbo, int& isum)
 {
-    const __half2 h01 = *reinterpret_cast<const __half2*>(&o.x), h23 = *reinterpret_cast<const __half2*>(&o.y);
-    const float hv[4] = {__low2float(h01), __high2float(h01), __low2float(h23), __high2float(h23)};
     // the block maximum in one warp reduction: non-negative floats order as their bit patterns do; a lane of NaNs counts
     // as 0 (fmaxf drops NaNs) unless every lane is one
     float amax = fmaxf(fmaxf(fabsf(hv[0]), fabsf(hv[1])), fmaxf(fabsf(hv[2]), fabsf(hv[3])));
@@ -356,13 +356,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
                     }
                     int pi, lbg;   // matrix of the stack, band group inside it
                     split_bg(gbg, pi, lbg);
-                    float sx;
+                    float sx, rot[4];
                     const uint2 o = rotate_block<false>(p.a + size_t(t) * p.k, p.het ? p.het_suh[pi] : p.suh + size_t(pi) * p.k, kb, lane, sx,
-                                                               p.a_up ? p.a_up + size_t(t) * p.k : nullptr, p.act_limit);
+                                                               p.a_up ? p.a_up + size_t(t) * p.k : nullptr, p.act_limit, rot);
                     int isum;
-                    const float scale = quantise_block(o, lane, area + size_t(j) * ftile + t * 32, 2 * flbo, flbo, isum);
+                    const float scale = quantise_block(rot, lane, area + size_t(j) * ftile + t * 32, 2 * flbo, flbo, isum);
                     if (lane == 0) {
-                        fscales[j * 8 + t] = scale;
+                        fscales[j * 8 + t] = 2.0f * scale;
                         fscales[j * 8 + 4 + t] = __fmul_rn(scale, __int2float_rn(isum));
                     }
                     if (lbg == 0) {   // band group 0 of a matrix meets every 128-block exactly once: the caller's copy
@@ -583,7 +583,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
                     sxp[t] = __fadd_rn(sxp[t], bs[t]);
 #pragma unroll
                     for (int b = 0; b < BU; ++b)
-                        acc[b][t] = __fmaf_rn(sc[t], __int2float_rn(r[b][2 * t] * 256 + r[b][2 * t + 1]), acc[b][t]);
+                        // half of 256 hi + lo, against twice the scale: the whole can pass 2^31 (a block whose rotated values are all
+                        // alike, as those of a one-hot input are), the half stays below 128 * 1020 * 127 * 128 + 2^23 < 2^31; the bit
+                        // that falls off is below the conversion's own rounding
+                        acc[b][t] = __fmaf_rn(sc[t], __int2float_rn(r[b][2 * t] * 128 + (r[b][2 * t + 1] >> 1)), acc[b][t]);
                 }
             }
             // ---- the segment's sums: thread et owns column et of every band
@@ -688,16 +691,16 @@ __global__ void __launch_bounds__(128) k_rotate_in_i8(const __half* __restrict__
     const int total = rows * kblocks;
     for (int idx = blockIdx.x * 4 + (threadIdx.x >> 5); idx < total; idx += gridDim.x * 4) {
         const int row = idx / kblocks, b = idx - row * kblocks;
-        float sx;
-        const uint2 o = rotate_block<false>(a + size_t(row) * k, suh, b, lane, sx, a_up ? a_up + size_t(row) * k : nullptr, act_limit);
+        float sx, rot[4];
+        const uint2 o = rotate_block<false>(a + size_t(row) * k, suh, b, lane, sx, a_up ? a_up + size_t(row) * k : nullptr, act_limit, rot);
         *reinterpret_cast<uint2*>(a_had + size_t(row) * k + b * 128 + lane * 4) = o;
         const size_t record = size_t(16) * nb * 256 + 128;          // limbs, then the block's scales (one per row)
         int isum;
-        const float scale = quantise_block(o, lane, limbs + size_t(b) * record + size_t(row >> 2) * 256 + (2 * (row & 3)) * 16, nb * 256, 128, isum);
+        const float scale = quantise_block(rot, lane, limbs + size_t(b) * record + size_t(row >> 2) * 256 + (2 * (row & 3)) * 16, nb * 256, 128, isum);
         if (lane == 0) {
             float* tail = reinterpret_cast<float*>(limbs + size_t(b) * record + size_t(16) * nb * 256);   // 16 scales, then 16 block sums
             const float bsum = __fmul_rn(scale, __int2float_rn(isum));
-            tail[row] = scale;
+            tail[row] = 2.0f * scale;
             tail[16 + row] = bsum;
             blocksum[size_t(row) * kblocks + b] = bsum;
         }

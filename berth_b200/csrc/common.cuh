@@ -234,8 +234,8 @@ std::string launch_gemv_i8(const void* a, const void* trellis, void* c, const vo
 std::string launch_gemv_i8_multi(const void* a, const void* const* trellis, void* const* c, const void* const* suh,
                                  void* const* a_had, const void* const* svh, const int* size_n, int n_matrices, int size_m,
                                  int size_k, int k_bits, int out_fp32, const GemvScratch& sc, int sms, cudaStream_t stream);
-// True when launch_gemv_i8 would rotate the activations inside the decode kernel for this dense shape.
-bool gemv_i8_rotates_in_kernel(int size_m, int size_k, int size_n, int k_bits, int sms);
+// True when launch_gemv hands this dense MUL1 linear to launch_gemv_i8.
+bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc);
 
 constexpr float kRScale = 0.088388347648f;  // 1/sqrt(128), csrc/prefill_lin/reconstruct.cu:43-44
 

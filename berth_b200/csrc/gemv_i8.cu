@@ -78,7 +78,10 @@ struct GeoI8 {
     static constexpr int PITCH = BU * 128 + 4;
     static constexpr int OUT_FLOATS = TOK * PITCH;
     static constexpr int D_COLS = 2 * BU * NCOL;               // two accumulator buffers
-    static constexpr int A_STAGE_COLS = BU * 64;               // half a unit: 4 k-tile rows x 16 columns per band
+    // Weight stage in tensor memory: half a unit of two bands, a whole unit of one -- 128 columns either way, so that a
+    // hand-over carries 16384 weights.
+    static constexpr int HALVES = BU == 2 ? 2 : 1, HROWS = 8 / HALVES;   // stages per unit, k-tile rows per stage
+    static constexpr int A_STAGE_COLS = BU * HROWS * 16;
     static constexpr int NA_RAW = (512 - D_COLS) / A_STAGE_COLS;
     static constexpr int NA = NA_RAW > 4 ? 4 : NA_RAW;
     static constexpr int kBarBytes = 512;
@@ -212,8 +215,7 @@ __device__ __forceinline__ float quantise_block(const float (&hv)[4], int lane, 
 }
 
 // ---------------------------------------------------------------- the kernel
-// FUSED (one group of four rows, dense launches in which no CTA holds a whole band group and every CTA's units fit
-// the limb area): no rotation kernel runs before this one and no limb tile travels through L2; while the first weight
+// FUSED (one group of four rows, dense launches in which the limb tiles of every CTA's units fit the limb area): no rotation kernel runs before this one and no limb tile travels through L2; while the first weight
 // stages are in flight the decoding and epilogue warps rotate and quantise the 128-block of every unit of the CTA
 // into a shared-memory area of its own (tiles of 2 * rows limb rows, a quarter of the ring-stage tile for one row),
 // and the CTAs that hold band group 0 also write the rotated activations and block sums for the caller and the
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
     constexpr int NW = G_::NW, BU = G_::BU, ROW_BYTES = G_::ROW_BYTES, W_BYTES = G_::W_BYTES, B_BYTES = G_::B_BYTES;
     constexpr int STAGE_BYTES = G_::STAGE_BYTES, S = G_::S, NA = G_::NA, TOK = ONE ? 1 : G_::TOK, NCOL = G_::NCOL, PITCH = G_::PITCH;
     constexpr int CHUNK_BYTES = G_::CHUNK_BYTES, A_STAGE_COLS = G_::A_STAGE_COLS, D_COLS = G_::D_COLS;
+    constexpr int HALVES = G_::HALVES, HROWS = G_::HROWS;
 
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -276,6 +279,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
     const long long u0 = unit_begin(cta, U, G), u1 = unit_begin(cta + 1, U, G);
     const int nunits = int(u1 - u0);
     const int gbg0 = int(u0 / kblocks), kb0 = int(u0 - (long long) gbg0 * kblocks);   // the CTA's first band group and 128-block
+    // FUSED: limb tiles of the CTA.  With one matrix a CTA of more units than the row has 128-blocks meets the same blocks
+    // again in its next band group: unit j uses tile j mod kblocks.
+    const int ntiles = nprob == 1 && nunits > kblocks ? kblocks : nunits;
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * S;
     const uint32_t afull0 = empty0 + 8 * S, aempty0 = afull0 + 8 * NA;
     const uint32_t dfull0 = aempty0 + 8 * NA, dempty0 = dfull0 + 16;
@@ -336,17 +342,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_d = s_tmem_base;             // accumulators: [buffer][band][NCOL]
-    const uint32_t tmem_a = tmem_d + D_COLS;         // weight stages: [NA][band][k-tile row of the half][16]
-    float* fscales = reinterpret_cast<float*>(area + size_t(nunits) * ftile + 512);   // FUSED: [unit][4 scales, 4 block sums]
+    const uint32_t tmem_a = tmem_d + D_COLS;         // weight stages: [NA][band][k-tile row of the stage][16]
+    float* fscales = reinterpret_cast<float*>(area + size_t(ntiles) * ftile + 512);   // FUSED: [tile][4 scales, 4 block sums]
 
     if constexpr (FUSED) {
         // In-kernel rotation: while the first weight stages are in flight, the decoding and the epilogue warps
-        // rotate and quantise the 128-block of every unit of the CTA (one warp per unit and row) into the limb area.
+        // rotate and quantise the 128-block of every tile of the CTA (one warp per tile and row) into the limb area.
         if (warp != kProducerWarp) {
             if (warp != kMmaWarp) {
                 pdl_wait();   // the activations come from the preceding kernels
                 const int w20 = warp;   // decode warps 0..15, epilogue warps 16..19
-                for (int task = w20; task < nunits * p.m; task += kDecodeWarps + kEpiWarps) {
+                for (int task = w20; task < ntiles * p.m; task += kDecodeWarps + kEpiWarps) {
                     const int j = p.m == 1 ? task : task / p.m, t = task - j * p.m;
                     int gbg = gbg0, kb = kb0 + j;   // unit u0 + j of the launch: no 64-bit division per task
                     if (kb >= kblocks) {
@@ -415,8 +421,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
         // ------------------------------------------------------------ decode warps
         const int quarter = warp & 3, stream = warp >> 2;
         const int band_l = BU == 2 ? (stream & 1) : 0;              // band of the unit this warp decodes
-        constexpr int NROWS = BU == 2 ? 2 : 1;                      // k-tile rows per warp and half-unit stage
-        const int r0 = BU == 2 ? 2 * (stream >> 1) : stream;        // first of them inside the half
+        constexpr int NROWS = 2;                                    // k-tile rows per warp and stage
+        const int r0 = BU == 2 ? 2 * (stream >> 1) : 2 * stream;    // first of them inside the stage
         const int lane1 = (lane + 1) & 31;
         // the warp's first tile inside a ring stage, and its first tensor-memory address inside a weight stage
         const int word0 = r0 * (ROW_BYTES / 4) + (band_l * 8 + 2 * quarter) * NW;
@@ -439,11 +445,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
             mbar_wait(full0 + 8 * s, phase, p.status, kStFullTimeout);   // (tight polling: a parked wait wakes up too late here)
             const uint32_t* stage = reinterpret_cast<const uint32_t*>(ring + s * STAGE_BYTES) + word0;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int h = 0; h < HALVES; ++h) {
                 const uint32_t taddr = taddr0 + a_idx * A_STAGE_COLS;
 #pragma unroll
                 for (int rr = 0; rr < NROWS; ++rr) {
-                    const uint32_t* rowp = stage + (4 * h + rr) * (ROW_BYTES / 4);
+                    const uint32_t* rowp = stage + (HROWS * h + rr) * (ROW_BYTES / 4);
                     uint32_t x[2][8];
 #pragma unroll
                     for (int t = 0; t < 2; ++t) {
@@ -478,17 +484,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
         // With one group of four rows the second group of eight limb rows the MMA asks for (N = 16) aliases the
         // next k-step's rows: those eight accumulator columns are never read.
         constexpr uint32_t kSbo = 256;
-        int s = 0, phase = 0, a_idx = 0, a_par = 0;
+        int s = 0, phase = 0, a_idx = 0, a_par = 0, tile = 0;
         for (int i = 0; i < nunits; ++i) {
             const int buf = i & 1;
             if constexpr (!FUSED) mbar_wait_suspended(full0 + 8 * s, phase, p.status, kStFullTimeout);   // the unit's limb tile has landed
             if (i >= 2) mbar_wait_suspended(dempty0 + 8 * buf, ((i >> 1) - 1) & 1, p.status, kStTmemTimeout);   // accumulator drained
-            const uint64_t b_desc0 = FUSED ? smem_desc_kmajor(smem_u32(area + size_t(i) * ftile), flbo, 2 * flbo)
+            const uint64_t b_desc0 = FUSED ? smem_desc_kmajor(smem_u32(area + size_t(tile) * ftile), flbo, 2 * flbo)
                                            : smem_desc_kmajor(smem_u32(ring + s * STAGE_BYTES + W_BYTES), 128, kSbo);
             const uint32_t chunk_step = FUSED ? uint32_t(2 * flbo) >> 4 : uint32_t(CHUNK_BYTES) >> 4;
             const uint32_t d_base = tmem_d + buf * (BU * NCOL);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int h = 0; h < HALVES; ++h) {
                 mbar_wait_suspended(afull0 + 8 * a_idx, a_par, p.status, kStTmemTimeout);
                 tc_fence_after();
                 const uint32_t a_base = tmem_a + a_idx * A_STAGE_COLS;
@@ -496,15 +502,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
 #pragma unroll
                     for (int b = 0; b < BU; ++b)
 #pragma unroll
-                        for (int r = 0; r < 4; ++r)
+                        for (int r = 0; r < HROWS; ++r)
 #pragma unroll
                             for (int j = 0; j < 2; ++j) {
-                                const int chunk = (4 * h + r) * 2 + j;
+                                const int chunk = (HROWS * h + r) * 2 + j;
                                 tc_mma_ts_i8(d_base + b * NCOL, a_base + b * 64 + r * 16 + 8 * j,
                                              b_desc0 + uint64_t(chunk * chunk_step), idesc, (h | r | j) ? 1u : 0u);
                             }
                     tc_commit(aempty0 + 8 * a_idx);
-                    if (h == 1) {
+                    if (h == HALVES - 1) {
                         tc_commit(dfull0 + 8 * buf);
                         if constexpr (!FUSED) tc_commit(empty0 + 8 * s);
                     }
@@ -513,6 +519,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
                 if (++a_idx == NA) { a_idx = 0; a_par ^= 1; }
             }
             if (++s == S) { s = 0; phase ^= 1; }
+            if (++tile == ntiles) tile = 0;
         }
     } else {
         // ------------------------------------------------------------ epilogue warps
@@ -525,7 +532,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
         const size_t slab_floats = size_t(slab_rows) * BU * 128;
         const size_t slab_stride = slab_floats + 32;          // ... followed by the rows' partial sums of the activations
         __shared__ int s_last;
-        int ui = 0, rs = 0, rphase = 0;
+        int ui = 0, tile = 0, rs = 0, rphase = 0;
         long long u = u0;
         while (u < u1) {
             const Segment sg = segment_at(u, u0, u1, kblocks);
@@ -551,9 +558,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
                 if constexpr (FUSED) {
 #pragma unroll
                     for (int t = 0; t < TOK; ++t) {
-                        sc[t] = t < rows ? fscales[ui * 8 + t] : 0.f;
-                        bs[t] = t < rows ? fscales[ui * 8 + 4 + t] : 0.f;
+                        sc[t] = t < rows ? fscales[tile * 8 + t] : 0.f;
+                        bs[t] = t < rows ? fscales[tile * 8 + 4 + t] : 0.f;
                     }
+                    if (++tile == ntiles) tile = 0;
                 } else {
                     // the unit's block scales and block sums travel with its limb tile
                     mbar_wait_suspended(full0 + 8 * rs, rphase, p.status, kStFullTimeout);
@@ -775,16 +783,19 @@ size_t launch_bits(int k_bits, int nb, bool fused, const void* const* t, int nm,
 
 }  // namespace
 
-bool gemv_i8_rotates_in_kernel(int size_m, int size_k, int size_n, int k_bits, int sms)
+// Whether launch_gemv sends a dense MUL1 linear here: the rotation fits the kernel and the scratch suffices (where it does
+// not, the fp16-path kernel still serves the shape).
+bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc)
 {
-    if (size_m < 1 || size_m > 4 || size_k % 128 != 0 || k_bits < 1 || k_bits > 8) return false;
+    if (size_m != 1 || size_k % 128 != 0 || size_n % 128 != 0 || k_bits < 1 || k_bits > 8) return false;
     const int bu = k_bits <= 4 ? 2 : 1;
     const int bands = size_n / 128, kblocks = size_k / 128, bgroups = (bands + bu - 1) / bu;
     const long long units = (long long) bgroups * kblocks;
     const int grid = int(std::min<long long>(std::min<long long>(sms, units), (long long) bgroups * 16));
-    if (grid < 1) return false;
-    const long long units_per_cta = (units + grid - 1) / grid;
-    return units_per_cta < kblocks && units_per_cta <= fused_max_units(k_bits, size_m <= 1 ? 1 : (size_m == 2 ? 2 : 4));
+    if (grid < 1 || std::min<long long>((units + grid - 1) / grid, kblocks) > fused_max_units(k_bits, size_m)) return false;
+    return size_t(bgroups) <= sc.counter_words && size_t(size_m) * kblocks <= sc.blocksum_floats &&
+           size_t(kblocks) * (size_t(16) * 256 + 128) <= sc.afrag_bytes &&
+           size_t(grid) * 2 * (size_t(size_m) * bu * 128 + 32) * sizeof(float) <= sc.slab_bytes;
 }
 
 // Rotation + decode linear for up to kI8MaxRows rows of a MUL1 matrix (or of a stack of n_stack equally shaped ones);
@@ -815,11 +826,12 @@ std::string launch_gemv_i8(const void* a, const void* trellis, void* c, const vo
     if (size_t(n_stack) * bgroups > sc.counter_words)
         throw std::runtime_error("exl3 gemv: matrices x size_n / 128 exceed the band-group counters of the scratch");
 
-    // In-kernel rotation for up to four rows when no CTA holds a whole band group (such a CTA finishes its bands
-    // itself and needs every block sum of the row, which other CTAs would still be writing).
-    const long long units_per_cta = (units + grid - 1) / grid;
+    // In-kernel rotation for up to four rows when the limb tiles a CTA meets fit its area: one per unit, and with one
+    // matrix never more than the row has 128-blocks.
+    long long tiles_per_cta = (units + grid - 1) / grid;
+    if (n_stack == 1) tiles_per_cta = std::min<long long>(tiles_per_cta, kblocks);
     const int frows = size_m <= 1 ? 1 : (size_m == 2 ? 2 : 4);
-    const bool fused = nb == 1 && units_per_cta < kblocks && units_per_cta <= fused_max_units(k_bits, frows);
+    const bool fused = nb == 1 && tiles_per_cta <= fused_max_units(k_bits, frows);
     const int rot_total = size_m * kblocks;
     if (!fused)
         for (int i = 0; i < n_stack; ++i)
@@ -899,7 +911,7 @@ std::string launch_gemv_i8_multi(const void* a, const void* const* trellis, void
     if (size_t(total_bg) > sc.counter_words) throw std::runtime_error("exl3 gemv: band groups exceed the counters of the scratch");
     const long long units_per_cta = (units + grid - 1) / grid;
     const int frows = size_m <= 1 ? 1 : (size_m == 2 ? 2 : 4);
-    const bool fused = nb == 1 && units_per_cta < kblocks && units_per_cta <= fused_max_units(k_bits, frows);
+    const bool fused = nb == 1 && units_per_cta <= fused_max_units(k_bits, frows);
     const int rot_total = size_m * kblocks;
     if (!fused)
         for (int i = 0; i < n_matrices; ++i)

@@ -234,6 +234,25 @@ std::string launch_gemv_i8(const void* a, const void* trellis, void* c, const vo
 std::string launch_gemv_i8_multi(const void* a, const void* const* trellis, void* const* c, const void* const* suh,
                                  void* const* a_had, const void* const* svh, const int* size_n, int n_matrices, int size_m,
                                  int size_k, int k_bits, int out_fp32, const GemvScratch& sc, int sms, cudaStream_t stream);
+// Grouped decode launch on the integer path with the rotation in the kernel (see GemvArgs for the row and scale rules).
+struct GroupedI8 {
+    const void* trellis;          // stack of n_matrices
+    const __half* src;            // input rows [.][k]; with src_up the input is silu(src) * src_up
+    const __half* src_up;
+    const __half *suh, *suh_b;
+    int z_half, row_half;
+    const int32_t* perm;
+    int div, n_perm, table_wait;
+    void* c;                      // fp16 rows [.][n]
+    const __half* svh;            // [n_matrices][n]
+    const GemvProblem* problems;
+    const int* n_problems;
+    int max_problems, n_matrices, max_rows;
+};
+bool gemv_i8_grouped_fits(long long most, int rows, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc);
+std::string launch_gemv_i8_grouped(const GroupedI8& g, int rows, int size_k, int size_n, int k_bits, const GemvScratch& sc, int sms,
+                                   cudaStream_t stream);
+
 // True when launch_gemv hands this dense MUL1 linear to launch_gemv_i8.
 bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc);
 

@@ -53,6 +53,13 @@ struct GemvArgs {
     const int* n_stride_list;
     const int* had_src_list;
     int n_slices;
+    // Grouped launch with the rotation in the kernel (integer tensor path only): row r of the problems (minus row_half from
+    // row_half on: the doubled table's second half) is row perm[r] / div of `a` for r < n_perm, row r - n_perm above; matrix z
+    // has its input scales at suh + z*k below z_half and at suh_b + (z - z_half)*k from there on.  table_wait: the problem
+    // table is written by the preceding kernel (no look at it before griddepcontrol.wait).
+    const __half* suh_b;
+    const int32_t* perm;
+    int div, n_perm, row_half, z_half, table_wait;
     // Stack of n_stack equally shaped matrices applied to the same rows (integer tensor path only; 0 or 1 = one
     // matrix): matrix i has its trellis at index i of the 3-D map, its sign-scale vectors at suh + i*k and
     // svh + i*n, and writes c + i*m*n, a_had + i*m*k and block sums i*m*(k/128).
@@ -77,7 +84,7 @@ struct ProblemView {
     void* c;                 // output base (row 0, column 0 of the problem)
     int ldc;                 // output row stride in elements
 };
-template <typename Args>
+template <typename Args, bool TABLE = true>   // TABLE = false: the caller knows that there is no problem table
 __device__ __forceinline__ ProblemView problem_view(const Args& p, int pi, int tok)
 {
     ProblemView v;
@@ -87,7 +94,7 @@ __device__ __forceinline__ ProblemView problem_view(const Args& p, int pi, int t
         v.svh = reinterpret_cast<const __half*>(__ldg(p.svh_list + pi));
         v.c = reinterpret_cast<void*>(__ldg(p.c_list + pi));
         v.ldc = __ldg(p.n_stride_list + pi);
-    } else if (p.problems) {
+    } else if (TABLE && p.problems) {
         const GemvProblem pr = load_problem(p.problems, pi, p.n_matrices, tok, p.max_rows);
         v.rows = pr.rows; v.row0 = pr.row0; v.z = pr.z; v.act = pi;
         v.svh = p.svh + size_t(pr.z) * p.n;

@@ -228,11 +228,15 @@ struct I8Maps {
 
 // ONE: the launch has one row (the epilogue warps then read two accumulator columns per band instead of eight and keep one
 // row's sums: they share their schedulers with the decode warps).
-template <int BITS, int NB, bool FUSED, bool ONE>
+// GROUPED: the band groups are those of a device-side problem table (the experts of an MoE layer); a template parameter
+// because every instruction of the dense launch's prologue is on its critical path (one 5120 x 6144 linear: 14.1 us, 14.5
+// with the table's branches in it).
+template <int BITS, int NB, bool FUSED, bool ONE, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_constant__ I8Maps maps, const GemvArgs p)
 {
     static_assert(!FUSED || NB == 1, "in-kernel rotation is built for one group of four rows");
     static_assert(!ONE || FUSED, "the one-row form exists for the in-kernel rotation only");
+    static_assert(!GROUPED || FUSED, "the grouped form rotates in the kernel");
     using G_ = GeoI8<BITS, NB, FUSED>;
     constexpr int NW = G_::NW, BU = G_::BU, ROW_BYTES = G_::ROW_BYTES, W_BYTES = G_::W_BYTES, B_BYTES = G_::B_BYTES;
     constexpr int STAGE_BYTES = G_::STAGE_BYTES, S = G_::S, NA = G_::NA, TOK = ONE ? 1 : G_::TOK, NCOL = G_::NCOL, PITCH = G_::PITCH;
@@ -250,11 +254,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
     const int frows = p.m <= 1 ? 1 : (p.m == 2 ? 2 : 4);
     const int flbo = 32 * frows, ftile = G_::fused_tile_bytes(frows);
 
+    if (GROUPED && p.table_wait) pdl_wait();   // (before the trigger: the next launch may read the same table ahead of its own wait)
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int bands = p.n >> 7, kblocks = p.k >> 7;
     const int bgroups = (bands + BU - 1) / BU;
-    const int nprob = p.problems ? min(max(__ldg(p.n_problems), 0), p.max_problems) : (p.n_stack > 1 ? p.n_stack : 1);
+    const int nprob = GROUPED ? min(max(__ldg(p.n_problems), 0), p.max_problems) : (p.n_stack > 1 ? p.n_stack : 1);
     const long long U = p.het ? (long long) p.het_bg[p.n_stack] * kblocks : (long long) nprob * bgroups * kblocks;
     // band group of the launch -> matrix and band group inside it
     auto split_bg = [&](int gbg, int& pi, int& lbg) {
@@ -296,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
     const int pre0 = pre < kPre0 ? pre : kPre0;
     constexpr uint32_t kStageTx = FUSED ? W_BYTES : STAGE_BYTES;
     auto issue_weights = [&](uint32_t dst, uint32_t bar) {
-        const int z = p.problems ? load_problem(p.problems, pr_pi, p.n_matrices, TOK, p.max_rows).z : (p.het ? 0 : pr_pi);
+        const int z = GROUPED ? load_problem(p.problems, pr_pi, p.n_matrices, TOK, p.max_rows).z : (p.het ? 0 : pr_pi);
         tma_load_3d(dst, &maps.m[p.het ? pr_pi : 0], pr_lbg * (ROW_BYTES / 8), pr_kb * 8, z, bar);
     };
     auto next_unit = [&]() {
@@ -362,16 +367,25 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
                     }
                     int pi, lbg;   // matrix of the stack, band group inside it
                     split_bg(gbg, pi, lbg);
+                    const __half* suh = p.het ? p.het_suh[pi] : p.suh + size_t(pi) * p.k;
+                    int src = t;
+                    if constexpr (GROUPED) {
+                        const GemvProblem pr = load_problem(p.problems, pi, p.n_matrices, TOK, p.max_rows);
+                        if (t >= pr.rows) continue;
+                        suh = pr.z < p.z_half ? p.suh + size_t(pr.z) * p.k : p.suh_b + size_t(pr.z - p.z_half) * p.k;
+                        const int r = pr.row0 + t - (pr.row0 >= p.row_half ? p.row_half : 0);
+                        src = r < p.n_perm ? min(max(__ldg(p.perm + r) / p.div, 0), max(p.n_perm / p.div - 1, 0)) : r - p.n_perm;
+                    }
                     float sx, rot[4];
-                    const uint2 o = rotate_block<false>(p.a + size_t(t) * p.k, p.het ? p.het_suh[pi] : p.suh + size_t(pi) * p.k, kb, lane, sx,
-                                                               p.a_up ? p.a_up + size_t(t) * p.k : nullptr, p.act_limit, rot);
+                    const uint2 o = rotate_block<false>(p.a + size_t(src) * p.k, suh, kb, lane, sx,
+                                                               p.a_up ? p.a_up + size_t(src) * p.k : nullptr, p.act_limit, rot);
                     int isum;
                     const float scale = quantise_block(rot, lane, area + size_t(j) * ftile + t * 32, 2 * flbo, flbo, isum);
                     if (lane == 0) {
                         fscales[j * 8 + t] = 2.0f * scale;
                         fscales[j * 8 + 4 + t] = __fmul_rn(scale, __int2float_rn(isum));
                     }
-                    if (lbg == 0) {   // band group 0 of a matrix meets every 128-block exactly once: the caller's copy
+                    if (lbg == 0 && !GROUPED) {   // band group 0 of a matrix meets every 128-block exactly once: the caller's copy
                         __half* ah = p.het ? p.het_a_had[pi] + size_t(t) * p.k : p.a_had + (size_t(pi) * p.m + t) * p.k;
                         *reinterpret_cast<uint2*>(ah + kb * 128 + lane * 4) = o;
                     }
@@ -538,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
             const Segment sg = segment_at(u, u0, u1, kblocks);
             int pi, lbg;
             split_bg(sg.bg, pi, lbg);
-            ProblemView pv = problem_view(p, pi, TOK);
+            ProblemView pv = problem_view<GemvArgs, GROUPED>(p, pi, TOK);
             if (p.het) {
                 pv.z = 0; pv.act = pi;
                 pv.svh = p.het_svh[pi]; pv.c = p.het_c[pi]; pv.ldc = p.het_n[pi];
@@ -730,11 +744,11 @@ int fused_max_units(int k_bits, int rows)
     }
 }
 
-template <int BITS, int NB, bool FUSED, bool ONE = false>
+template <int BITS, int NB, bool FUSED, bool ONE = false, bool GROUPED = false>
 size_t launch_one(const void* const* trellis, int n_matrices, const GemvArgs& args, int grid, cudaStream_t stream)
 {
     using G_ = GeoI8<BITS, NB, FUSED>;
-    auto kern = k_exl3_gemv_i8<BITS, NB, FUSED, ONE>;
+    auto kern = k_exl3_gemv_i8<BITS, NB, FUSED, ONE, GROUPED>;
     static bool attr_set[kMaxDevices] = {};
     const int dev = current_device();
     if (!attr_set[dev]) {
@@ -760,6 +774,7 @@ size_t launch_nb(int nb, bool fused, const void* const* t, int nm, const GemvArg
 {
     switch (nb) {
         case 1:
+            if (a.problems) return a.m == 1 ? launch_one<BITS, 1, true, true, true>(t, nm, a, grid, st) : launch_one<BITS, 1, true, false, true>(t, nm, a, grid, st);
             if (fused) return a.m == 1 ? launch_one<BITS, 1, true, true>(t, nm, a, grid, st) : launch_one<BITS, 1, true>(t, nm, a, grid, st);
             return launch_one<BITS, 1, false>(t, nm, a, grid, st);
         default: return launch_one<BITS, 2, false>(t, nm, a, grid, st);
@@ -937,6 +952,51 @@ std::string launch_gemv_i8_multi(const void* a, const void* const* trellis, void
     return std::string(fused ? "" : "k_rotate_in_i8 + ") + "k_exl3_gemv_i8<" + std::to_string(k_bits) + "," + std::to_string(nb) +
            (fused ? ",fused" : "") + "," + std::to_string(n_matrices) + " matrices> grid=" + std::to_string(grid) + " block=" +
            std::to_string(kThreads) + " smem=" + std::to_string(smem);
+}
+
+// Grouped decode launch of a few rows (at most four per problem) with the rotation in the kernel and the split-K sums
+// finished by the last CTA to arrive: one launch where the fp16-path form takes three (rotation, decode, finishing
+// kernel).  `most` = most problems the table can hold for these rows; the table itself is on the device.
+bool gemv_i8_grouped_fits(long long most, int rows, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc)
+{
+    if (rows < 1 || rows > 4 || size_k % 128 != 0 || size_n % 128 != 0 || most < 1) return false;
+    const int bu = k_bits <= 4 ? 2 : 1;
+    const long long bgroups = (size_n / 128 + bu - 1) / bu, units = most * bgroups * (size_k / 128);
+    const size_t per_cta = size_t(2) * (size_t(rows) * bu * 128 + 32) * sizeof(float);
+    return (units + sms - 1) / sms <= fused_max_units(k_bits, rows <= 1 ? 1 : (rows == 2 ? 2 : 4)) && size_t(most * bgroups) <= sc.counter_words &&
+           size_t(sms) * per_cta <= sc.slab_bytes;
+}
+
+std::string launch_gemv_i8_grouped(const GroupedI8& g, int rows, int size_k, int size_n, int k_bits, const GemvScratch& sc, int sms,
+                                   cudaStream_t stream)
+{
+    GemvArgs args{};
+    args.defer_weights = weights_streamed() ? 1 : 0;
+    args.a = g.src;
+    args.a_up = g.src_up;
+    args.suh = g.suh;
+    args.suh_b = g.suh_b;
+    args.z_half = g.z_half;
+    args.row_half = g.row_half;
+    args.perm = g.perm;
+    args.div = g.div;
+    args.n_perm = g.n_perm;
+    args.table_wait = g.table_wait;
+    args.c = g.c;
+    args.svh = g.svh;
+    args.problems = g.problems;
+    args.n_problems = g.n_problems;
+    args.max_problems = g.max_problems;
+    args.n_matrices = g.n_matrices;
+    args.max_rows = g.max_rows;
+    args.slabs = sc.slabs;
+    args.counters = sc.counters;
+    args.status = sc.status;
+    args.m = rows; args.k = size_k; args.n = size_n;
+    args.out_fp32 = 0;
+    const size_t smem = launch_bits(k_bits, 1, true, &g.trellis, g.n_matrices, args, sms, stream);
+    return "k_exl3_gemv_i8<" + std::to_string(k_bits) + ",1,fused,grouped> grid=" + std::to_string(sms) + " block=" + std::to_string(kThreads) +
+           " smem=" + std::to_string(smem);
 }
 
 }  // namespace berth

@@ -934,6 +934,8 @@ struct RowSource {
     const int32_t* perm = nullptr;
     int div = 1, n_perm = 0;
     bool paired = false;   // the problem table was written twice (scan_problems, pair_rows = max_rows) and up lies behind gate
+    int rows_per_problem = 0;   // > 0: no problem has more rows than this (few tokens), and the table holds at most `most`
+    long long most = 0;
 };
 
 // Grouped gate/up -> silu*up -> down over routed rows xr [R][hidden]; yr fp16 [R][hidden].
@@ -982,6 +984,44 @@ std::string experts(const berth_moe_weights* w, const void* gate_t, const void* 
                                        H, w->k_bits, w->codebook, 0, sc.status, sms, st);
         return std::string("k_rotate_rows_plain<gate+up> + ") + (paired ? "1 x (gate and up as one stack) " : "2 x ") + d +
                " + k_rotate_rows_plain<silu> + 1 x (same, down)";
+    }
+    // A few tokens (at most four rows per expert), MUL1: the integer-path kernel rotates in the launch and finishes in it, so the
+    // stage is two launches; the fp16-path form below is six, and at this size every launch costs its latency (an A3B layer
+    // of one token: 56 us that way, 41 this way).
+    if (src.rows_per_problem > 0 && w->codebook == 2 &&
+        gemv_i8_grouped_fits((paired ? 2 : 1) * src.most, src.rows_per_problem, H, I, w->k_bits, sms, sc) &&
+        gemv_i8_grouped_fits(src.most, src.rows_per_problem, I, H, w->k_bits, sms, sc)) {
+        const int m = src.rows_per_problem;
+        GroupedI8 g{};
+        g.trellis = gate_t;
+        g.src = static_cast<const __half*>(xr);
+        g.suh = static_cast<const __half*>(gsuh); g.suh_b = static_cast<const __half*>(usuh);
+        g.z_half = n_local; g.row_half = max_rows;
+        g.perm = src.perm; g.div = src.div; g.n_perm = src.n_perm;
+        g.table_wait = 1;
+        g.c = s.g; g.svh = static_cast<const __half*>(gsvh);
+        g.problems = s.problems; g.n_problems = s.n_problems + (paired ? 1 : 0);
+        g.max_problems = int((paired ? 2 : 1) * src.most);
+        g.n_matrices = (paired ? 2 : 1) * n_local; g.max_rows = (paired ? 2 : 1) * max_rows;
+        const std::string d = launch_gemv_i8_grouped(g, m, H, I, w->k_bits, sc, sms, st);
+        if (!paired) {
+            g.trellis = up_t;
+            g.suh = static_cast<const __half*>(usuh);
+            g.table_wait = 0;
+            g.c = s.u; g.svh = static_cast<const __half*>(usvh);
+            launch_gemv_i8_grouped(g, m, H, I, w->k_bits, sc, sms, st);
+        }
+        GroupedI8 gd{};
+        gd.trellis = down_t;
+        gd.src = s.g; gd.src_up = u_out;
+        gd.suh = static_cast<const __half*>(dsuh);
+        gd.z_half = n_local; gd.row_half = max_rows;
+        gd.div = 1;
+        gd.c = yr; gd.svh = static_cast<const __half*>(dsvh);
+        gd.problems = s.problems; gd.n_problems = s.n_problems;
+        gd.max_problems = int(src.most); gd.n_matrices = n_local; gd.max_rows = max_rows;
+        launch_gemv_i8_grouped(gd, m, I, H, w->k_bits, sc, sms, st);
+        return std::string(paired ? "1 x (gate and up as one stack: " : "2 x (") + d + ") + 1 x (same, down, silu in the rotation)";
     }
     const int tg = plan.tg;
     RotateFragArgs r{};
@@ -1106,9 +1146,14 @@ extern "C" int berth_moe_experts(const berth_moe_weights* w, const void* xr, voi
         if (info.major != 10) throw std::runtime_error("moe experts: no linked kernel for this GPU (library is built for sm_100a only)");
         ExpertScratch es = expert_scratch(ews, ews_bytes, max_rows, w->n_experts, w->hidden, w->inter, max_rows_per_expert);
         if (n_rows == 0) return;
+        RowSource in_place{};
+        if (n_rows <= 4) {   // as the layer does; at most as many problems as rows
+            in_place.rows_per_problem = n_rows;
+            in_place.most = std::min(n_rows, w->n_experts);
+        }
         st.launch = experts(w, w->gate_trellis, w->up_trellis, w->down_trellis, w->gate_suh, w->gate_svh, w->up_suh, w->up_svh,
                             w->down_suh, w->down_svh, w->n_experts, xr, yr, n_rows, n_rows, expert_plan(max_rows_per_expert), es,
-                            gemv_workspace(device), info.sms, (cudaStream_t) stream);
+                            gemv_workspace(device), info.sms, (cudaStream_t) stream, nullptr, in_place);
     });
 }
 
@@ -1221,6 +1266,10 @@ extern "C" int berth_moe_ep_experts(const berth_moe_weights* w, const void* recv
         }
         RowSource in_place{};
         in_place.paired = up_behind_gate(w, NM);
+        if (n_rows + TS > 0 && std::max(n_rows, TS) <= 4) {   // as the layer does
+            in_place.rows_per_problem = std::max(n_rows, TS);
+            in_place.most = std::min(n_rows, NL) + (TS ? 1 : 0);
+        }
         dispatch(keys, n_rows, 0, NL, plan.chunk, es, perm, inv, cs, TS, in_place.paired ? RT : 0, NM);
         if (n_rows > 0) {
             launch_pdl(k_moe_gather_rows, dim3(std::min(n_rows, 148 * 8)), dim3(256), 0, cs, "k_moe_gather_rows launch", (const __half*) recv_rows, perm, es.offsets + NL, 1, xr, H);
@@ -1375,6 +1424,10 @@ extern "C" int berth_moe_p2p_experts(const berth_moe_weights* w, const void* x_l
         __half* xr = static_cast<__half*>(pr.p[rank]);
         RowSource in_place{};
         in_place.paired = up_behind_gate(w, NM);
+        if (world == 1 && T_local >= 1 && T_local <= 4) {   // (more ranks: how many rows arrive is known on the device only)
+            in_place.rows_per_problem = T_local;
+            in_place.most = std::min(T_local * top_k, NL) + (TS ? 1 : 0);
+        }
         launch_pdl(k_moe_scan, dim3(1), dim3(1024), 0, cs, "k_moe_scan launch", es.counts, es.offsets, es.problems, es.n_problems, NL, plan.chunk, TS,
                    in_place.paired ? max_rows : 0, NM, es.max_problems, max_rows, sc.status);
         cuda_ok(cudaGetLastError(), "k_moe_scan launch");
@@ -1457,6 +1510,10 @@ extern "C" int berth_moe_layer(const berth_moe_weights* w, const void* x, int T,
         RowSource rows_from{};
         rows_from.perm = perm; rows_from.div = K; rows_from.n_perm = R;
         rows_from.paired = paired;
+        if (T <= 4) {   // a token goes to an expert once: at most T rows per problem, at most one problem per expert hit
+            rows_from.rows_per_problem = T;
+            rows_from.most = std::min(R, E) + (fused_shared ? 1 : 0);
+        }
         st.launch = experts(w, w->gate_trellis, w->up_trellis, w->down_trellis, w->gate_suh, w->gate_svh, w->up_suh, w->up_svh,
                             w->down_suh, w->down_svh, NM, x, yr, RT, RT, plan, es, sc, info.sms, cs, nullptr, rows_from);
 

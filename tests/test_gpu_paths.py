@@ -5,8 +5,8 @@ import pytest
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-from berth_b200 import kernels, synth   # noqa: E402
-from tests.gpu_util import assert_close, run_linear   # noqa: E402
+from berth_b200 import kernels, moe, synth   # noqa: E402
+from tests.gpu_util import assert_close, dev, run_linear   # noqa: E402
 
 
 def test_integer_path_one_hot_blocks(oracle):
@@ -31,3 +31,23 @@ def test_integer_path_several_band_groups_per_cta(oracle, K, N, bits):
     assert "k_exl3_gemv_i8" in kernels.last_launch() and "fused" in kernels.last_launch()
     assert_close(c, oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, 2), "wide")
     assert kernels.device_status(torch.cuda.current_device()) == 0
+
+@pytest.mark.parametrize("T", [1, 2, 3, 4, 5, 9])
+@pytest.mark.parametrize("bits,inter,shared,E", [(4, 128, 128, 32), (3, 384, 384, 64), (5, 256, 0, 32)])
+def test_moe_layer_few_tokens_vs_oracle(oracle, T, bits, inter, shared, E):
+    """One launch per projection (up to four tokens) and the grouped decode launches above, gate and up as one stack and
+    apart, the shared expert inside the stacks, apart and absent."""
+    H, k = 512, 8
+    wts = synth.moe_layer_weights(1234, f"few{bits}", H, inter, E, k, bits, 2, shared_inter=shared)
+    x = synth.activations(1234, f"few.x{T}", T, H)
+    for pair, fuse in ((True, True), (False, False)):
+        layer = moe.MoeLayer(torch.device("cuda"), wts, T, fuse_shared=fuse, pair_gate_up=pair)
+        out = torch.full((T, H), float("nan"), dtype=torch.float32, device="cuda")
+        idx = torch.empty((T, k), dtype=torch.int32, device="cuda")
+        w = torch.empty((T, k), dtype=torch.float32, device="cuda")
+        layer.forward(dev(x), out, idx, w)
+        torch.cuda.synchronize()
+        assert kernels.device_status(torch.cuda.current_device()) == 0
+        _, exp_idx, exp_w = oracle.moe_layer(wts, x)
+        assert (idx.cpu().numpy() == exp_idx).all()
+        assert_close(out.cpu().numpy(), oracle.moe_layer_f64(wts, x, exp_idx, exp_w), f"T={T} pair={pair}")

@@ -23,19 +23,22 @@ namespace {
 // compared bit for bit.  Block = 16 warps x 32 experts for kRouterTok tokens: a warp accumulates
 // chunks j and j+16 with coalesced reads of the router rows (each row read once per token tile).
 constexpr int kRouterTok = 8;
-// The halving tree over the 32 chunk sums, p[c] at base[c * kRouterTok * 33]: V(c, 32) = p[c],
+// The halving tree over the 32 chunk sums, p[c] at base[c * TOK * 33]: V(c, 32) = p[c],
 // V(c, s) = V(c, 2s) + V(c + s, 2s), result V(0, 1) -- evaluated depth first, a handful of registers.
-template <int S>
+template <int S, int TOK>
 __device__ __forceinline__ float chunk_tree(const float* base, int c)
 {
-    if constexpr (S == 32) return base[c * (kRouterTok * 33)];
-    else return __fadd_rn(chunk_tree<2 * S>(base, c), chunk_tree<2 * S>(base, c + S));
+    if constexpr (S == 32) return base[c * (TOK * 33)];
+    else return __fadd_rn(chunk_tree<2 * S, TOK>(base, c), chunk_tree<2 * S, TOK>(base, c + S));
 }
-// Dynamic shared memory: the token tile as fp32 [kRouterTok][H], then the chunk sums [32][kRouterTok][33].
+// Dynamic shared memory: the token tile as fp32 [TOK][H], then the chunk sums [32][TOK][33].
 // WARPS = 16: each warp accumulates two of the 32 chunks, one after the other; 512 threads and ~97 KiB per block,
 // so that two blocks share an SM and one block's load and reduction phases overlap the other's arithmetic.
 // WARPS = 32: one chunk per warp, for launches of fewer blocks than SMs, which the latency of a chunk's loads bounds.
-template <int WARPS>
+// TOK = tokens per block.  A launch of fewer blocks than SMs takes the fewest tokens per block that still fit one wave:
+// its multiply-adds and shared-memory reads (and, for one token, eight times the work for rows that do not exist) were
+// most of its time; with TOK <= 2 the registers also hold 32 router rows in flight instead of 8.
+template <int WARPS, int TOK>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 2 : 1) k_moe_router_logits(const __half* __restrict__ x, const __half* __restrict__ w,
                                                                             const float* __restrict__ bias, float* __restrict__ logits,
                                                                             int T, int H, int E)
@@ -43,14 +46,14 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 2 : 1) k_moe_router_
     pdl_trigger();   // launched as a programmatic dependent: let the successor become resident, then wait for the predecessor
     pdl_wait();
     extern __shared__ __align__(16) float rsm[];
-    float* xs = rsm;                                                    // [kRouterTok][H]
-    float (*part)[kRouterTok][33] = reinterpret_cast<float (*)[kRouterTok][33]>(rsm + kRouterTok * H);
+    float* xs = rsm;                                                    // [TOK][H]
+    float (*part)[TOK][33] = reinterpret_cast<float (*)[TOK][33]>(rsm + TOK * H);
     const int wq = threadIdx.x >> 5, el = threadIdx.x & 31;
-    const int e = blockIdx.x * 32 + el, t0 = blockIdx.y * kRouterTok;
+    const int e = blockIdx.x * 32 + el, t0 = blockIdx.y * TOK;
     const int chunk = H / 32;
     // the tile's activations, converted once (rows past T repeat the last token; their sums are never stored)
-    for (int i = threadIdx.x * 2; i < kRouterTok * H; i += WARPS * 64) {
-        const int tt = i / H, h = i - tt * H;
+    for (int i = threadIdx.x * 2; i < TOK * H; i += WARPS * 64) {
+        const int tt = TOK == 1 ? 0 : i / H, h = i - tt * H;
         const __half2 v = *reinterpret_cast<const __half2*>(x + size_t(min(t0 + tt, T - 1)) * H + h);
         xs[i] = __low2float(v);
         xs[i + 1] = __high2float(v);
@@ -60,16 +63,32 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 2 : 1) k_moe_router_
     for (int j = wq; j < 32; j += WARPS) {
         const __half* wr = w + size_t(j) * chunk * E + e;
         const float* xj = xs + j * chunk;
-        float acc[kRouterTok];
+        float acc[TOK];
 #pragma unroll
-        for (int tt = 0; tt < kRouterTok; ++tt) acc[tt] = 0.f;
+        for (int tt = 0; tt < TOK; ++tt) acc[tt] = 0.f;
         // eight router rows in flight per pass, the next eight already requested; the products are still
         // added one by one in k order
         int i0 = 0;
-        __half nxt[8];
-        if (8 <= vec_end) {
+        if constexpr (TOK <= 2) {
+            for (; i0 + 32 <= vec_end; i0 += 32) {
+                __half wv[32];
 #pragma unroll
-            for (int ii = 0; ii < 8; ++ii) nxt[ii] = wr[size_t(ii) * E];
+                for (int ii = 0; ii < 32; ++ii) wv[ii] = wr[size_t(i0 + ii) * E];
+#pragma unroll
+                for (int ii = 0; ii < 32; ii += 4) {
+#pragma unroll
+                    for (int tt = 0; tt < TOK; ++tt) {
+                        const float4 a = *reinterpret_cast<const float4*>(xj + tt * H + i0 + ii);
+                        acc[tt] = __fmaf_rn(a.x, __half2float(wv[ii]), acc[tt]); acc[tt] = __fmaf_rn(a.y, __half2float(wv[ii + 1]), acc[tt]);
+                        acc[tt] = __fmaf_rn(a.z, __half2float(wv[ii + 2]), acc[tt]); acc[tt] = __fmaf_rn(a.w, __half2float(wv[ii + 3]), acc[tt]);
+                    }
+                }
+            }
+        }
+        __half nxt[8];
+        if (i0 + 8 <= vec_end) {
+#pragma unroll
+            for (int ii = 0; ii < 8; ++ii) nxt[ii] = wr[size_t(i0 + ii) * E];
         }
         for (; i0 + 8 <= vec_end; i0 += 8) {
             float wv[8];
@@ -80,7 +99,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 2 : 1) k_moe_router_
                 for (int ii = 0; ii < 8; ++ii) nxt[ii] = wr[size_t(i0 + 8 + ii) * E];
             }
 #pragma unroll
-            for (int tt = 0; tt < kRouterTok; ++tt) {
+            for (int tt = 0; tt < TOK; ++tt) {
                 const float4 a = *reinterpret_cast<const float4*>(xj + tt * H + i0);
                 const float4 b = *reinterpret_cast<const float4*>(xj + tt * H + i0 + 4);
                 acc[tt] = __fmaf_rn(a.x, wv[0], acc[tt]); acc[tt] = __fmaf_rn(a.y, wv[1], acc[tt]);
@@ -92,15 +111,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 2 : 1) k_moe_router_
         for (; i0 < chunk; ++i0) {   // the rest, or all of it for an odd chunk
             const float wv = __half2float(wr[size_t(i0) * E]);
 #pragma unroll
-            for (int tt = 0; tt < kRouterTok; ++tt) acc[tt] = __fmaf_rn(xj[tt * H + i0], wv, acc[tt]);
+            for (int tt = 0; tt < TOK; ++tt) acc[tt] = __fmaf_rn(xj[tt * H + i0], wv, acc[tt]);
         }
 #pragma unroll
-        for (int tt = 0; tt < kRouterTok; ++tt) part[j][tt][el] = acc[tt];
+        for (int tt = 0; tt < TOK; ++tt) part[j][tt][el] = acc[tt];
     }
     __syncthreads();
     // warp tt reduces token tt: lane = expert; the same halving tree as a 32-lane xor butterfly's lane 0
-    if (wq < kRouterTok && t0 + wq < T) {
-        logits[size_t(t0 + wq) * E + e] = __fadd_rn(chunk_tree<1>(&part[0][wq][el], 0), bias ? bias[e] : 0.f);
+    if (wq < TOK && t0 + wq < T) {
+        logits[size_t(t0 + wq) * E + e] = __fadd_rn(chunk_tree<1, TOK>(&part[0][wq][el], 0), bias ? bias[e] : 0.f);
     }
 }
 
@@ -202,6 +221,7 @@ __global__ void __launch_bounds__(512, 1) k_moe_router_logits_wide(const __half*
 }
 
 // One warp per token: k rounds of arg-max, value descending then index ascending.
+template <int PER>   // experts per lane: E <= 32 * PER
 __global__ void __launch_bounds__(128) k_moe_topk(const float* __restrict__ logits, int32_t* __restrict__ topk_idx,
                                                   float* __restrict__ topk_w, int T, int E, int k)
 {
@@ -210,41 +230,48 @@ __global__ void __launch_bounds__(128) k_moe_topk(const float* __restrict__ logi
     const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= T) return;
     const float* l = logits + size_t(t) * E;
-    constexpr int kMaxPerLane = 32;   // E <= 1024
-    float v[kMaxPerLane];
-    const int per = (E + 31) / 32;
+    // key of an expert: the order-preserving bits of its logit (-0 counts as +0), 0 for a NaN and for one already taken.
+    // A lane keeps its best key, and only the lane that lost it looks through its PER experts again; the row's best is one
+    // warp maximum over the keys and one minimum over the indices that have it.
+    auto key_of = [](float v) {
+        const uint32_t b = __float_as_uint(__fadd_rn(v, 0.0f));
+        return v != v ? 0u : ((b & 0x80000000u) ? ~b : (b | 0x80000000u));
+    };
+    float v[PER];
 #pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) v[i] = (i < per && lane + 32 * i < E) ? l[lane + 32 * i] : -INFINITY;
-    unsigned taken = 0;   // bit i: this lane's i-th expert already selected
+    for (int i = 0; i < PER; ++i) v[i] = lane + 32 * i < E ? l[lane + 32 * i] : 0.f;
+    unsigned taken = 0;   // bit i: this lane's i-th expert is selected (or past the row)
+#pragma unroll
+    for (int i = 0; i < PER; ++i) taken |= lane + 32 * i < E ? 0u : 1u << i;
+    unsigned best = 0;
+    int best_i = 0;
+    auto look = [&]() {
+        best = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const unsigned key = (taken >> i) & 1u ? 0u : key_of(v[i]);
+            if (key > best) { best = key; best_i = i; }
+        }
+    };
+    look();
     float first = 0.f, mine = 0.f, sum = 0.f;
     for (int s = 0; s < k; ++s) {
+        const unsigned top = __reduce_max_sync(dq::kFull, best);
+        int bi;
         float bv = -INFINITY;
-        int bi = 0x7fffffff;
-#pragma unroll
-        for (int i = 0; i < kMaxPerLane; ++i)
-            if (i < per && !((taken >> i) & 1u) && lane + 32 * i < E) {
-                const int idx = lane + 32 * i;
-                if (v[i] > bv || (v[i] == bv && idx < bi)) { bv = v[i]; bi = idx; }
-            }
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) {
-            const float ov = __shfl_xor_sync(dq::kFull, bv, off);
-            const int oi = __shfl_xor_sync(dq::kFull, bi, off);
-            if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+        if (top != 0u) {
+            bi = int(__reduce_min_sync(dq::kFull, best == top ? unsigned(lane + 32 * best_i) : 0xffffffffu));
+            bv = __uint_as_float((top & 0x80000000u) ? (top & 0x7fffffffu) : ~top);
+        } else {
+            // nothing left of the row but NaN: take the lowest expert not selected yet, so that the k indices are always
+            // distinct and inside [0, E): the dispatch and combine kernels index arrays with them.
+            const unsigned left = ~taken & (PER == 32 ? 0xffffffffu : (1u << (PER & 31)) - 1u);
+            bi = int(__reduce_min_sync(dq::kFull, left ? unsigned(lane + 32 * (__ffs(left) - 1)) : 0xffffffffu));
         }
-        if (bi == 0x7fffffff) {
-            // nothing compared greater than -inf: what is left of the row is NaN (or the row is all -inf).  Take the lowest
-            // expert not selected yet, so that the k indices are always distinct and inside [0, E): the dispatch and
-            // combine kernels index arrays with them.
-            int fi = 0x7fffffff;
-#pragma unroll
-            for (int i = kMaxPerLane - 1; i >= 0; --i)
-                if (i < per && !((taken >> i) & 1u) && lane + 32 * i < E) fi = lane + 32 * i;
-#pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) fi = min(fi, __shfl_xor_sync(dq::kFull, fi, off));
-            bi = fi;
+        if ((bi & 31) == lane) {
+            taken |= 1u << (bi >> 5);
+            look();
         }
-        if ((bi & 31) == lane) taken |= 1u << (bi >> 5);
         if (s == 0) first = bv;
         const float ex = expf(bv - first);
         sum += ex;
@@ -880,16 +907,22 @@ void router_topk(const void* x, const void* w_router, const float* bias, int32_t
 {
     const size_t smem = size_t(kRouterTok) * H * 4 + size_t(32) * kRouterTok * 33 * 4;
     if (smem > 200 * 1024) throw std::runtime_error("moe router: hidden is too large for the router's shared-memory tile");
+    const int dev = current_device(), sms = device_info(dev).sms;
     static bool attr_set[kMaxDevices] = {};
-    const int dev = current_device();
     if (!attr_set[dev]) {
-        cuda_ok(cudaFuncSetAttribute(k_moe_router_logits<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), "router smem attribute");
-        cuda_ok(cudaFuncSetAttribute(k_moe_router_logits<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), "router smem attribute");
+        for (auto kern : {k_moe_router_logits<32, 1>, k_moe_router_logits<32, 2>, k_moe_router_logits<32, 4>, k_moe_router_logits<32, 8>, k_moe_router_logits<16, 8>})
+            cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), "router smem attribute");
         attr_set[dev] = true;
     }
     const dim3 rgrid(E / 32, (T + kRouterTok - 1) / kRouterTok);
     const size_t smem_wide = size_t(kRouterTok) * H * 4 + size_t(16) * kRouterTok * kWidePitch * 4;
-    if (E % 128 == 0 && H % 256 == 0 && smem_wide <= 200 * 1024 && int(rgrid.x * rgrid.y) > 2 * device_info(dev).sms) {
+    auto narrow = [&](auto kern, int warps, int tok) {
+        const size_t bytes = size_t(tok) * H * 4 + size_t(32) * tok * 33 * 4;
+        launch_pdl(kern, dim3(E / 32, (T + tok - 1) / tok), dim3(warps * 32), bytes, st, "k_moe_router_logits launch", (const __half*) x,
+                   (const __half*) w_router, bias, logits, T, H, E);
+    };
+    auto one_wave = [&](int tok) { return (long long) (E / 32) * ((T + tok - 1) / tok) <= sms; };
+    if (E % 128 == 0 && H % 256 == 0 && smem_wide <= 200 * 1024 && int(rgrid.x * rgrid.y) > 2 * sms) {
         static bool wide_set[kMaxDevices] = {};
         if (!wide_set[dev]) {
             cuda_ok(cudaFuncSetAttribute(k_moe_router_logits_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), "router smem attribute");
@@ -897,14 +930,13 @@ void router_topk(const void* x, const void* w_router, const float* bias, int32_t
         }
         launch_pdl(k_moe_router_logits_wide, dim3(E / 128, rgrid.y), dim3(512), smem_wide, st, "k_moe_router_logits_wide launch",
                    (const __half*) x, (const __half*) w_router, bias, logits, T, H, E);
-    } else if (int(rgrid.x * rgrid.y) <= device_info(dev).sms)
-        launch_pdl(k_moe_router_logits<32>, rgrid, dim3(32 * 32), smem, st, "k_moe_router_logits launch", (const __half*) x,
-                   (const __half*) w_router, bias, logits, T, H, E);
-    else
-        launch_pdl(k_moe_router_logits<16>, rgrid, dim3(16 * 32), smem, st, "k_moe_router_logits launch", (const __half*) x,
-                   (const __half*) w_router, bias, logits, T, H, E);
+    } else if (one_wave(1)) narrow(k_moe_router_logits<32, 1>, 32, 1);
+    else if (one_wave(2)) narrow(k_moe_router_logits<32, 2>, 32, 2);
+    else if (one_wave(4)) narrow(k_moe_router_logits<32, 4>, 32, 4);
+    else if (one_wave(8)) narrow(k_moe_router_logits<32, 8>, 32, 8);
+    else narrow(k_moe_router_logits<16, 8>, 16, 8);
     cuda_ok(cudaGetLastError(), "k_moe_router_logits launch");
-    launch_pdl(k_moe_topk, dim3((T + 3) / 4), dim3(128), 0, st, "k_moe_topk launch", logits, topk_idx, topk_w, T, E, k);
+    launch_pdl(E <= 128 ? k_moe_topk<4> : (E <= 256 ? k_moe_topk<8> : k_moe_topk<32>), dim3((T + 3) / 4), dim3(128), 0, st, "k_moe_topk launch", logits, topk_idx, topk_w, T, E, k);
     cuda_ok(cudaGetLastError(), "k_moe_topk launch");
 }
 

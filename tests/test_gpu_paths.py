@@ -51,3 +51,20 @@ def test_moe_layer_few_tokens_vs_oracle(oracle, T, bits, inter, shared, E):
         _, exp_idx, exp_w = oracle.moe_layer(wts, x)
         assert (idx.cpu().numpy() == exp_idx).all()
         assert_close(out.cpu().numpy(), oracle.moe_layer_f64(wts, x, exp_idx, exp_w), f"T={T} pair={pair}")
+
+@pytest.mark.parametrize("T", [1, 2, 18, 19, 37, 75, 150])
+@pytest.mark.parametrize("H,E", [(2048, 256), (96, 64), (1056, 512)])
+def test_router_tiles_bit_exact(oracle, T, H, E):
+    """Every token tile of the router (one, two, four, eight tokens per block; the row remainders of its unrolled loops)."""
+    k = 8
+    x, w = synth.activations(1234, f"rt.x{T}", T, H), synth.router_weight(1234, f"rt{H}", H, E)
+    idx = torch.empty((T, k), dtype=torch.int32, device="cuda")
+    tw = torch.empty((T, k), dtype=torch.float32, device="cuda")
+    logits = torch.empty((T, E), dtype=torch.float32, device="cuda")
+    moe.router_topk(dev(x), dev(w), None, idx, tw, logits, T, H, E, k)
+    torch.cuda.synchronize()
+    exp_logits = oracle.router_logits(x, w)
+    exp_idx, exp_w = oracle.router_topk(exp_logits, k)
+    assert (logits.cpu().numpy().view(np.uint32) == exp_logits.view(np.uint32)).all()
+    assert (idx.cpu().numpy() == exp_idx).all()
+    assert np.abs(tw.cpu().numpy() - exp_w).max() <= 1e-6

@@ -61,7 +61,7 @@ constexpr int kSmemBudget = 227 * 1024;
 
 // Compile-time geometry: BITS bits per weight, NB groups of four rows (two limb columns each); FUSED = the
 // limb tiles of all the CTA's units live in a shared-memory area of their own instead of the ring stages.
-template <int BITS, int NB, bool FUSED>
+template <int BITS, int NB, bool FUSED, bool ONE>
 struct GeoI8 {
     static constexpr int NW = 8 * BITS;
     static constexpr int BU = BITS <= 4 ? 2 : 1;
@@ -86,12 +86,15 @@ struct GeoI8 {
     static constexpr int NA = NA_RAW > 4 ? 4 : NA_RAW;
     static constexpr int kBarBytes = 512;
     static constexpr int RING_MAX = kSmemBudget - 1024 - OUT_FLOATS * 4 - kBarBytes - 64;
-    static constexpr int kMinArea = 80 * 1024;                 // in-kernel rotation: least size of the limb area
+    // in-kernel rotation: least size of the limb area.  Above one row it takes what a deeper weight ring would: about 96 KiB
+    // of weights in flight cover the memory latency, and three rows of a CTA's 37 units (gate and up of a 5120 x 17408 MLP
+    // as one launch) need 112 KiB of tiles.
+    static constexpr int kMinArea = (ONE ? 80 : 128) * 1024;
     static constexpr int S_RAW = (RING_MAX - (FUSED ? kMinArea : 0)) / STAGE_BYTES;
     static constexpr int S = S_RAW > 12 ? 12 : S_RAW;
     static constexpr int AREA_BYTES = FUSED ? RING_MAX - S * STAGE_BYTES : 0;
     static constexpr size_t SMEM = 1024 + size_t(S) * STAGE_BYTES + OUT_FLOATS * 4 + kBarBytes + AREA_BYTES;
-    // in-kernel rotation: a unit's limb tile holds 2*rows limb rows per core matrix (rows = 1, 2 or 4), core
+    // in-kernel rotation: a unit's limb tile holds 2*rows limb rows per core matrix (rows = 1 to 4), core
     // matrices 32*rows bytes apart, 16 k-steps of two core matrices, plus four scales and four block sums; 512 bytes of the area stay
     // free because the MMA reads whole 8-row core matrices (the rows past 2*rows are never used)
     __host__ __device__ static constexpr int fused_tile_bytes(int rows) { return 1024 * rows; }
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
     static_assert(!FUSED || NB == 1, "in-kernel rotation is built for one group of four rows");
     static_assert(!ONE || FUSED, "the one-row form exists for the in-kernel rotation only");
     static_assert(!GROUPED || FUSED, "the grouped form rotates in the kernel");
-    using G_ = GeoI8<BITS, NB, FUSED>;
+    using G_ = GeoI8<BITS, NB, FUSED, ONE>;
     constexpr int NW = G_::NW, BU = G_::BU, ROW_BYTES = G_::ROW_BYTES, W_BYTES = G_::W_BYTES, B_BYTES = G_::B_BYTES;
     constexpr int STAGE_BYTES = G_::STAGE_BYTES, S = G_::S, NA = G_::NA, TOK = ONE ? 1 : G_::TOK, NCOL = G_::NCOL, PITCH = G_::PITCH;
     constexpr int CHUNK_BYTES = G_::CHUNK_BYTES, A_STAGE_COLS = G_::A_STAGE_COLS, D_COLS = G_::D_COLS;
@@ -251,7 +254,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
     unsigned char* area = reinterpret_cast<unsigned char*>(bars) + G_::kBarBytes;   // FUSED: limb tiles, then four scales per unit
     __shared__ uint32_t s_tmem_base;
     // FUSED: limb rows per core matrix = 2 * frows, core matrices frows * 32 bytes apart
-    const int frows = p.m <= 1 ? 1 : (p.m == 2 ? 2 : 4);
+    const int frows = ONE ? 1 : p.m;
     const int flbo = 32 * frows, ftile = G_::fused_tile_bytes(frows);
 
     if (GROUPED && p.table_wait) pdl_wait();   // (before the trigger: the next launch may read the same table ahead of its own wait)
@@ -730,24 +733,29 @@ __global__ void __launch_bounds__(128) k_rotate_in_i8(const __half* __restrict__
 }
 
 // Most units per CTA whose limb tiles fit the limb area of the in-kernel rotation.
+template <int BITS>
+int fused_max_units(int rows)
+{
+    return rows == 1 ? GeoI8<BITS, 1, true, true>::fused_max_units(1) : GeoI8<BITS, 1, true, false>::fused_max_units(rows);
+}
 int fused_max_units(int k_bits, int rows)
 {
     switch (k_bits) {
-        case 1: return GeoI8<1, 1, true>::fused_max_units(rows);
-        case 2: return GeoI8<2, 1, true>::fused_max_units(rows);
-        case 3: return GeoI8<3, 1, true>::fused_max_units(rows);
-        case 4: return GeoI8<4, 1, true>::fused_max_units(rows);
-        case 5: return GeoI8<5, 1, true>::fused_max_units(rows);
-        case 6: return GeoI8<6, 1, true>::fused_max_units(rows);
-        case 7: return GeoI8<7, 1, true>::fused_max_units(rows);
-        default: return GeoI8<8, 1, true>::fused_max_units(rows);
+        case 1: return fused_max_units<1>(rows);
+        case 2: return fused_max_units<2>(rows);
+        case 3: return fused_max_units<3>(rows);
+        case 4: return fused_max_units<4>(rows);
+        case 5: return fused_max_units<5>(rows);
+        case 6: return fused_max_units<6>(rows);
+        case 7: return fused_max_units<7>(rows);
+        default: return fused_max_units<8>(rows);
     }
 }
 
 template <int BITS, int NB, bool FUSED, bool ONE = false, bool GROUPED = false>
 size_t launch_one(const void* const* trellis, int n_matrices, const GemvArgs& args, int grid, cudaStream_t stream)
 {
-    using G_ = GeoI8<BITS, NB, FUSED>;
+    using G_ = GeoI8<BITS, NB, FUSED, ONE>;
     auto kern = k_exl3_gemv_i8<BITS, NB, FUSED, ONE, GROUPED>;
     static bool attr_set[kMaxDevices] = {};
     const int dev = current_device();
@@ -802,7 +810,7 @@ size_t launch_bits(int k_bits, int nb, bool fused, const void* const* t, int nm,
 // not, the fp16-path kernel still serves the shape).
 bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc)
 {
-    if (size_m != 1 || size_k % 128 != 0 || size_n % 128 != 0 || k_bits < 1 || k_bits > 8) return false;
+    if (size_m < 1 || size_m > 4 || size_k % 128 != 0 || size_n % 128 != 0 || k_bits < 1 || k_bits > 8) return false;
     const int bu = k_bits <= 4 ? 2 : 1;
     const int bands = size_n / 128, kblocks = size_k / 128, bgroups = (bands + bu - 1) / bu;
     const long long units = (long long) bgroups * kblocks;
@@ -845,8 +853,7 @@ std::string launch_gemv_i8(const void* a, const void* trellis, void* c, const vo
     // matrix never more than the row has 128-blocks.
     long long tiles_per_cta = (units + grid - 1) / grid;
     if (n_stack == 1) tiles_per_cta = std::min<long long>(tiles_per_cta, kblocks);
-    const int frows = size_m <= 1 ? 1 : (size_m == 2 ? 2 : 4);
-    const bool fused = nb == 1 && tiles_per_cta <= fused_max_units(k_bits, frows);
+    const bool fused = nb == 1 && tiles_per_cta <= fused_max_units(k_bits, size_m);
     const int rot_total = size_m * kblocks;
     if (!fused)
         for (int i = 0; i < n_stack; ++i)
@@ -925,8 +932,7 @@ std::string launch_gemv_i8_multi(const void* a, const void* const* trellis, void
     if (grid < 1) throw std::runtime_error("exl3 gemv: split-K scratch is too small for this shape");
     if (size_t(total_bg) > sc.counter_words) throw std::runtime_error("exl3 gemv: band groups exceed the counters of the scratch");
     const long long units_per_cta = (units + grid - 1) / grid;
-    const int frows = size_m <= 1 ? 1 : (size_m == 2 ? 2 : 4);
-    const bool fused = nb == 1 && units_per_cta <= fused_max_units(k_bits, frows);
+    const bool fused = nb == 1 && units_per_cta <= fused_max_units(k_bits, size_m);
     const int rot_total = size_m * kblocks;
     if (!fused)
         for (int i = 0; i < n_matrices; ++i)
@@ -963,7 +969,7 @@ bool gemv_i8_grouped_fits(long long most, int rows, int size_k, int size_n, int 
     const int bu = k_bits <= 4 ? 2 : 1;
     const long long bgroups = (size_n / 128 + bu - 1) / bu, units = most * bgroups * (size_k / 128);
     const size_t per_cta = size_t(2) * (size_t(rows) * bu * 128 + 32) * sizeof(float);
-    return (units + sms - 1) / sms <= fused_max_units(k_bits, rows <= 1 ? 1 : (rows == 2 ? 2 : 4)) && size_t(most * bgroups) <= sc.counter_words &&
+    return (units + sms - 1) / sms <= fused_max_units(k_bits, rows) && size_t(most * bgroups) <= sc.counter_words &&
            size_t(sms) * per_cta <= sc.slab_bytes;
 }
 

@@ -32,6 +32,16 @@ def test_integer_path_several_band_groups_per_cta(oracle, K, N, bits):
     assert_close(c, oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, 2), "wide")
     assert kernels.device_status(torch.cuda.current_device()) == 0
 
+@pytest.mark.parametrize("m", [2, 3, 4])
+@pytest.mark.parametrize("K,N,bits", [(5120, 1024, 4), (2176, 3072, 5), (128, 128 * 301, 6), (1152, 640, 3)])
+def test_integer_path_two_to_four_rows(oracle, m, K, N, bits):
+    w = synth.linear_weights(1234, f"few{K}{bits}", K, N, bits)
+    x = synth.activations(1234, f"few{K}.x{m}", m, K)
+    c, ah = run_linear(x, w, bits, 2, False)
+    assert "k_exl3_gemv_i8" in kernels.last_launch()
+    assert_close(c, oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, 2), "few rows")
+    assert (ah == oracle.had_r_128(x, w["suh"], True).view(np.uint16)).all()
+
 @pytest.mark.parametrize("T", [1, 2, 3, 4, 5, 9])
 @pytest.mark.parametrize("bits,inter,shared,E", [(4, 128, 128, 32), (3, 384, 384, 64), (5, 256, 0, 32)])
 def test_moe_layer_few_tokens_vs_oracle(oracle, T, bits, inter, shared, E):

@@ -56,6 +56,12 @@ constexpr long long kWaitCycles = 500000000LL;
 
 enum : unsigned { kStGemmTimeout = 16u };
 
+// Epilogue of the dense kernel, over the idle rings: per team a transposition buffer (32 rows of 129 floats) and the band's
+// scales; behind them, for a tile whose K is split over a cluster, exchange buffers of one pass each (32 rows x 128 columns).
+constexpr int kEpiTeams = 5, kXchPitch = 129, kXchFloats = 32 * kXchPitch;
+constexpr int kXbufSlotBytes = 32 * 128 * 4, kXbufSlots = 7;
+constexpr int kSplitEpilogueBytes = kEpiTeams * (kXchFloats + 128) * 4 + kXbufSlots * kXbufSlotBytes;
+
 template <int BITS>
 struct TGeo {
     static constexpr int NW = 8 * BITS;
@@ -67,7 +73,10 @@ struct TGeo {
     static constexpr int kEpilogueExtra = (32 * 129 + 2 * 128) * 4;
     static constexpr int kFree = 227 * 1024 - 1024 - SA * A_STAGE_BYTES - kEpilogueExtra - kBarrierBytes - 2048 /*static shared*/;
     static constexpr int ST = kFree / T_STAGE_BYTES < 4 ? 4 : (kFree / T_STAGE_BYTES > 16 ? 16 : kFree / T_STAGE_BYTES);
-    static constexpr size_t SMEM = 1024 /*align slack*/ + size_t(SA) * A_STAGE_BYTES + size_t(ST) * T_STAGE_BYTES + kBarrierBytes;
+    static constexpr int RINGS = SA * A_STAGE_BYTES + ST * T_STAGE_BYTES;
+    static constexpr int DENSE_RINGS = RINGS > kSplitEpilogueBytes ? RINGS : kSplitEpilogueBytes;   // (the dense kernel's epilogue lies over them)
+    static constexpr size_t SMEM = 1024 /*align slack*/ + size_t(DENSE_RINGS) + kBarrierBytes;
+    static_assert(SMEM + 2048 <= 227 * 1024, "shared memory");
 };
 
 struct GemmArgs {
@@ -79,6 +88,8 @@ struct GemmArgs {
     const GemvProblem* problems;   // grouped launch: one entry per (matrix, chunk of <= nsub_max*128 rows); else null
     const int* n_problems;
     int max_problems, n_matrices;
+    int split;          // dense launch: CTAs of a cluster along z that share a tile's K (1 = the tile is one CTA's)
+    int defer_weights;  // no weight fetch before griddepcontrol.wait (berth_exl3_weights_streamed)
     int epi2;   // grouped launch with 128-row problems and a short K: two epilogue teams and three decode groups (see the kernel)
 };
 
@@ -217,7 +228,28 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr)
     d |= uint64_t(2) << 61;                      // SWIZZLE_128B
     return d;
 }
-constexpr int kEpiTeams = 5;
+// ---- clusters (a tile whose K is split)
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Barrier of all threads of the cluster's CTAs; what was written before it (to any of their shared memories) is seen after it.
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, uint32_t rank)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
 // Barrier of one epilogue team (four warps); ids 1..5.
 __device__ __forceinline__ void team_sync(int team) { asm volatile("bar.sync %0, 128;" ::"r"(team + 1) : "memory"); }
 // True in exactly one lane of a converged warp.
@@ -236,8 +268,6 @@ __device__ __forceinline__ bool elect_one()
 // 128-point Hadamard over n with ascending strides: 1..16 in registers, 32 and 64 between the four
 // threads of a row by shuffles (sgn * v + o is o - v or v + o, rounded once); then the output scale
 // (svh_s: the band's 128 scales as fp32) and 16-byte stores of rows row0 .. row0+31 below row_end.
-constexpr int kXchPitch = 129;
-constexpr int kXchFloats = 32 * kXchPitch;
 __device__ __forceinline__ void epilogue_rows(float (&v)[32], float* xch, const float* svh_s, int team, int quarter, int lane, void* c,
                                               int out_fp32, int ldc, int col0, int row0, int row_end)
 {
@@ -363,13 +393,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
     const int nsub = (rows_here + SUB - 1) / SUB;
     const int rows_pad = (rows_here + 15) & ~15;          // MMA N granularity
     const int n1 = min(rows_pad, 256), n2 = rows_pad - n1;   // rows of the first / second MMA of a k step
-    const int kstages = p.k / BK;
+    // the CTA's share of K (all of it unless the tile's K is split over the CTAs of a cluster)
+    const int k0 = p.k / BK * int(blockIdx.z) / p.split, kstages = p.k / BK * (int(blockIdx.z) + 1) / p.split - k0;
 
+    pdl_trigger();
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* a_ring = smem;
     unsigned char* t_ring = a_ring + SA * A_STAGE_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(t_ring + ST * T_STAGE_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TG_::DENSE_RINGS);
     __shared__ uint32_t s_tmem_base;
 
     const uint32_t full_a = smem_u32(bars), empty_a = full_a + 8 * SA;
@@ -400,17 +432,26 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_t) : "memory");
             int sa = 0, pa = 0, st = 0, pt = 0;
-            for (int ks = 0; ks < kstages; ++ks) {
-                // raw trellis: 4 k-tile rows of this band
-                if (ks >= ST) mbar_wait_parked(empty_t + 8 * st, pt ^ 1, p.status, 100);
+            auto load_trellis = [&](int ks) {   // 4 k-tile rows of this band
                 mbar_arrive_expect_tx(full_t + 8 * st, T_STAGE_BYTES);
-                tma_load_3d(smem_u32(t_ring + st * T_STAGE_BYTES), &tmap_t, band * (TROW_BYTES / 8), ks * 4, z, full_t + 8 * st);
+                tma_load_3d(smem_u32(t_ring + st * T_STAGE_BYTES), &tmap_t, band * (TROW_BYTES / 8), (k0 + ks) * 4, z, full_t + 8 * st);
                 if (++st == ST) { st = 0; pt ^= 1; }
+            };
+            // the weights do not depend on the rotation kernel: the first lap of the ring is requested before the wait for it
+            const int pre = min(kstages, ST);
+            if (p.defer_weights) pdl_wait();
+            for (int ks = 0; ks < pre; ++ks) load_trellis(ks);
+            pdl_wait();
+            for (int ks = 0; ks < kstages; ++ks) {
+                if (ks >= ST) {
+                    mbar_wait_parked(empty_t + 8 * st, pt ^ 1, p.status, 100);
+                    load_trellis(ks);
+                }
                 // activations: nsub boxes of 128 rows x 64 k (rows past the array read as zero)
                 if (ks >= SA) mbar_wait_parked(empty_a + 8 * sa, pa ^ 1, p.status, 100);
                 mbar_arrive_expect_tx(full_a + 8 * sa, nsub * A_SUB_BYTES);
                 for (int sub = 0; sub < nsub; ++sub)
-                    tma_load_2d(smem_u32(a_ring + sa * A_STAGE_BYTES + sub * A_SUB_BYTES), &tmap_a, ks * BK, m0 + sub * SUB,
+                    tma_load_2d(smem_u32(a_ring + sa * A_STAGE_BYTES + sub * A_SUB_BYTES), &tmap_a, (k0 + ks) * BK, m0 + sub * SUB,
                                 full_a + 8 * sa);
                 if (++sa == SA) { sa = 0; pa ^= 1; }
             }
@@ -481,10 +522,49 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
         float* svh_s = xch + kXchFloats;
         svh_s[n] = scale;
         team_sync(team);
-        for (int c0 = 32 * team; c0 < rows_pad; c0 += 32 * kEpiTeams)
-            epilogue_pass(tmem + (uint32_t(quarter * 32) << 16) + c0, xch, svh_s, team, quarter, lane, p.c, p.out_fp32, p.n, band * BN,
-                          m0 + c0, row_end);
-        tc_fence_before();
+        if (p.split == 1) {
+            for (int c0 = 32 * team; c0 < rows_pad; c0 += 32 * kEpiTeams)
+                epilogue_pass(tmem + (uint32_t(quarter * 32) << 16) + c0, xch, svh_s, team, quarter, lane, p.c, p.out_fp32, p.n, band * BN,
+                              m0 + c0, row_end);
+            tc_fence_before();
+        }
+    }
+    if (p.split > 1) {
+        // K split: pass i (32 rows) is finished by CTA i % split of the cluster.  The others leave their sums of it in that
+        // CTA's shared memory (behind the epilogue's own buffers, where the rings were: kXbufSlots passes of 16 KiB), and it
+        // adds them to its own in a fixed order.
+        const int S = p.split, me = int(cluster_rank()), quarter = warp & 3, n = quarter * 32 + lane;
+        const uint32_t tacc = tmem + (uint32_t(quarter * 32) << 16);
+        unsigned char* xbuf = a_ring + kEpiTeams * (kXchFloats + 128) * 4;
+        float v[32];
+        __syncwarp();
+        cluster_sync();   // every CTA's accumulator is complete, so every ring is idle
+        if (team >= 0)
+            for (int i = team; 32 * i < rows_pad; i += kEpiTeams) {
+                const int owner = i % S;
+                if (owner == me) continue;
+                tc_ld32(tacc + 32 * i, v);
+                const int slot = (i / S) * (S - 1) + (me < owner ? me : me - 1);
+                const uint32_t dst = cluster_addr(smem_u32(xbuf + slot * kXbufSlotBytes) + 4 * n, owner);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) cluster_store(dst + 512 * j, v[j]);
+            }
+        __syncwarp();
+        cluster_sync();   // the sums are where they are added up
+        if (team >= 0) {
+            float* xch = reinterpret_cast<float*>(a_ring) + team * (kXchFloats + 128);
+            for (int q = team; 32 * (me + q * S) < rows_pad; q += kEpiTeams) {
+                const int c0 = 32 * (me + q * S);
+                tc_ld32(tacc + c0, v);
+                for (int o = 0; o < S - 1; ++o) {
+                    const float* src = reinterpret_cast<const float*>(xbuf + (q * (S - 1) + o) * kXbufSlotBytes) + n;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = __fadd_rn(v[j], src[128 * j]);
+                }
+                epilogue_rows(v, xch, xch + kXchFloats, team, quarter, lane, p.c, p.out_fp32, p.n, band * BN, m0 + c0, row_end);
+            }
+            tc_fence_before();
+        }
     }
 
     __syncthreads();
@@ -503,7 +583,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
 template <int BITS>
 struct GGeo {
     static constexpr int T_STAGE_BYTES = TGeo<BITS>::T_STAGE_BYTES;
-    static constexpr size_t SMEM = TGeo<BITS>::SMEM + (kXchFloats + 2 * 128) * 4 /*transposition buffer and scales of the epilogue*/;
+    static constexpr size_t SMEM = 1024 + size_t(TGeo<BITS>::RINGS) + kBarrierBytes + (kXchFloats + 2 * 128) * 4 /*transposition buffer and scales of the epilogue*/;
 };
 
 // Three views of the activations (boxes of 32, 64 and 128 rows x 64 k): an item loads only as many rows as
@@ -1120,9 +1200,19 @@ void launch_tc(const void* a_had, const void* trellis, const GemmArgs& args, cud
         cuda_ok(cudaGetLastError(), "k_exl3_gemm_tc_grouped launch");
         return;
     }
-    dim3 grid(args.n / BN, (args.m + args.nsub_max * SUB - 1) / (args.nsub_max * SUB));
-    kern<<<grid, kThreads, TG_::SMEM, stream>>>(map_a, map_t, args);
-    cuda_ok(cudaGetLastError(), "k_exl3_gemm_tc launch");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(args.n / BN, (args.m + args.nsub_max * SUB - 1) / (args.nsub_max * SUB), args.split);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = TG_::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = unsigned(args.split);
+    cfg.attrs = attr;
+    cfg.numAttrs = args.split > 1 ? 2 : 1;
+    cuda_ok(cudaLaunchKernelEx(&cfg, kern, map_a, map_t, args), "k_exl3_gemm_tc launch");
 }
 
 template <int BITS>
@@ -1326,25 +1416,41 @@ std::string launch_gemm_tc(const void* a, const void* trellis, void* c, const vo
     args.out_fp32 = out_fp32;
     args.problems = nullptr; args.n_problems = nullptr; args.max_problems = 0; args.n_matrices = 1;
     args.epi2 = 0;
-    // Rows per CTA: 128, 256 or 384.  More rows per decoded weight keep the kernel MMA bound, fewer rows give
-    // more CTAs; pick the count with the least (waves x time of one CTA), the latter from the measured stage
-    // and epilogue times of the three tile heights (ns per 64-deep stage; ns per epilogue; 1.2 us to start).
+    args.defer_weights = weights_streamed() ? 1 : 0;
+    // Rows per CTA (128, 256 or 384) and CTAs that share a tile's K (1 to 8, a cluster).  More rows per decoded weight keep
+    // the kernel MMA bound, fewer rows or a split K give more CTAs; pick the pair with the least (waves x time of one CTA),
+    // the latter from the measured stage and epilogue times of the three tile heights (ns per 64-deep stage; ns per
+    // epilogue; 1.2 us to start; a split adds the exchange of the sums and two cluster barriers, and a CTA keeps at least
+    // four stages).  Without the split a 5120 x 1024 projection of 421 rows ran on 16 SMs and a 17408 x 5120 one on 80
+    // (a layer's chunk of 421 rows, together with the programmatic launch: 620 -> 541 us; 40 rows of a 2560-wide layer: 242 -> 105 us).
+    args.nsub_max = 1;
+    args.split = 1;
     {
         static const int kStageNs[MAX_SUB] = {430, 490, 540}, kEpilogueNs[MAX_SUB] = {4000, 7400, 10300};
         const int sms = device_info(current_device()).sms;
-        const int bands = size_n / BN;
+        const int bands = size_n / BN, stages = size_k / BK;
         long long best = -1;
-        for (int ns = 1; ns <= MAX_SUB; ++ns) {
-            const long long ctas = (long long) bands * ((size_m + ns * SUB - 1) / (ns * SUB));
-            const long long waves = (ctas + sms - 1) / sms;
-            const long long cost = waves * ((long long) (size_k / BK) * kStageNs[ns - 1] + kEpilogueNs[ns - 1] + 1200);
-            if (best < 0 || cost <= best) { best = cost; args.nsub_max = ns; }   // ties: more rows per CTA
-        }
+        for (int ns = 1; ns <= MAX_SUB; ++ns)
+            for (int sp = 1; sp == 1 || (sp <= 8 && 4 * sp <= stages); ++sp) {
+                const int passes = (std::min(size_m, ns * SUB) + 31) / 32;
+                if ((passes + sp - 1) / sp * (sp - 1) > kXbufSlots) continue;
+                // a cluster lies inside one of the eight GPCs
+                const long long slots = sp == 1 ? sms : std::max(sp, 8 * (sms / 8 / sp * sp));
+                const long long ctas = (long long) bands * ((size_m + ns * SUB - 1) / (ns * SUB)) * sp;
+                const long long waves = (ctas + slots - 1) / slots;
+                const long long epilogue = sp == 1 ? kEpilogueNs[ns - 1] : kEpilogueNs[ns - 1] / sp + 4000;
+                const long long cost = waves * ((long long) ((stages + sp - 1) / sp) * kStageNs[ns - 1] + epilogue + 1200);
+                if (best < 0 || cost < best || (cost == best && sp == 1)) {   // ties: more rows per CTA
+                    best = cost;
+                    args.nsub_max = ns;
+                    args.split = sp;
+                }
+            }
     }
     launch_tc_bits(k_bits, codebook, a_had, trellis, args, stream);
     return "k_had128<f16,pre> + k_exl3_gemm_tc<" + std::to_string(k_bits) + "," + std::to_string(codebook) + "> grid=" +
            std::to_string(size_n / BN) + "x" + std::to_string((size_m + args.nsub_max * SUB - 1) / (args.nsub_max * SUB)) +
-           " block=" + std::to_string(kThreads) + " tile=" + std::to_string(args.nsub_max * SUB) + "x128x64 tmem=512";
+           (args.split > 1 ? "x" + std::to_string(args.split) : "") + " block=" + std::to_string(kThreads) + " tile=" + std::to_string(args.nsub_max * SUB) + "x128x64 tmem=512";
 }
 
 // Decode batches of up to 32 rows on the tensor-core path: rotate the rows, then the persistent split-K kernel.
@@ -1416,6 +1522,8 @@ std::string launch_gemm_tc_grouped_rotated(const void* xr_had, const void* trell
     args.out_fp32 = out_fp32;
     args.nsub_max = nsub;
     args.problems = problems; args.n_problems = n_problems; args.max_problems = max_problems; args.n_matrices = n_matrices;
+    args.split = 1;
+    args.defer_weights = 0;
     // a main loop of at most sixteen stages is shorter than the epilogue of a 128-row item
     args.epi2 = (nsub == 1 && size_k <= 1024) ? 1 : 0;
     launch_tc_bits(k_bits, codebook, xr_had, trellis_stack, args, stream);

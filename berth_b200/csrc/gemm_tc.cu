@@ -1400,6 +1400,33 @@ __global__ void __launch_bounds__(256) k_rotate_rows_plain(const RotateArgs a)
 void had_r_128(const void* input, void* output, const void* scale, int pre_scale, int rows, int cols, int fp32,
                cudaStream_t stream);
 
+// CTAs of the dense kernel that run at once in clusters of `size` (0: such a cluster does not fit).  A cluster lies inside one
+// GPC, and how many SMs a GPC has differs: a B200 of 148 SMs does not hold 16 clusters of eight (their extra wave made a 421-row
+// 5120 x 1024 projection 30 us, clusters of four 20 us), so the driver is asked, once per device and size.
+static int cluster_slots(int size)
+{
+    const int dev = current_device();
+    if (size == 1) return device_info(dev).sms;
+    static int known[kMaxDevices][9] = {};   // slots + 1
+    if (!known[dev][size]) {
+        auto kern = k_exl3_gemm_tc<4, 2>;    // (every instance takes a whole SM)
+        cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TGeo<4>::SMEM)), "gemm smem attribute");
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, 1, size);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = TGeo<4>::SMEM;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = unsigned(size);
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        cuda_ok(cudaOccupancyMaxActiveClusters(&n, kern, &cfg), "cluster occupancy");
+        known[dev][size] = n * size + 1;
+    }
+    return known[dev][size] - 1;
+}
+
 // Prefill linear for any row count > 32: rotate the activations, then the tensor-core GEMM.
 std::string launch_gemm_tc(const void* a, const void* trellis, void* c, const void* suh, void* a_had, const void* svh,
                            int size_m, int size_k, int size_n, int k_bits, int codebook, int out_fp32, unsigned* status,
@@ -1422,20 +1449,19 @@ std::string launch_gemm_tc(const void* a, const void* trellis, void* c, const vo
     // the latter from the measured stage and epilogue times of the three tile heights (ns per 64-deep stage; ns per
     // epilogue; 1.2 us to start; a split adds the exchange of the sums and two cluster barriers, and a CTA keeps at least
     // four stages).  Without the split a 5120 x 1024 projection of 421 rows ran on 16 SMs and a 17408 x 5120 one on 80
-    // (a layer's chunk of 421 rows, together with the programmatic launch: 620 -> 541 us; 40 rows of a 2560-wide layer: 242 -> 105 us).
+    // (a layer's chunk of 421 rows, together with the programmatic launch: 620 -> 517 us; 40 rows of a 2560-wide layer: 242 -> 105 us).
     args.nsub_max = 1;
     args.split = 1;
     {
         static const int kStageNs[MAX_SUB] = {430, 490, 540}, kEpilogueNs[MAX_SUB] = {4000, 7400, 10300};
-        const int sms = device_info(current_device()).sms;
         const int bands = size_n / BN, stages = size_k / BK;
         long long best = -1;
         for (int ns = 1; ns <= MAX_SUB; ++ns)
             for (int sp = 1; sp == 1 || (sp <= 8 && 4 * sp <= stages); ++sp) {
                 const int passes = (std::min(size_m, ns * SUB) + 31) / 32;
                 if ((passes + sp - 1) / sp * (sp - 1) > kXbufSlots) continue;
-                // a cluster lies inside one of the eight GPCs
-                const long long slots = sp == 1 ? sms : std::max(sp, 8 * (sms / 8 / sp * sp));
+                const long long slots = cluster_slots(sp);
+                if (slots < 1) continue;
                 const long long ctas = (long long) bands * ((size_m + ns * SUB - 1) / (ns * SUB)) * sp;
                 const long long waves = (ctas + slots - 1) / slots;
                 const long long epilogue = sp == 1 ? kEpilogueNs[ns - 1] : kEpilogueNs[ns - 1] / sp + 4000;

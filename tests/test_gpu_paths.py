@@ -95,3 +95,16 @@ def test_prefill_split_k(oracle, m, K, N, bits, cb, out_fp32):
         again, _ = run_linear(x, w, bits, cb, out_fp32, prefill=True)
         assert again.tobytes() == c.tobytes()
     assert kernels.device_status(torch.cuda.current_device()) == 0
+
+
+@pytest.mark.parametrize("rows,K,skip", [(421, 5120, 0), (74, 128 * 128, 0), (9473, 128, 0), (3159, 384, 0), (421, 5120, 4)])
+def test_rotation_of_many_rows_bit_exact(oracle, rows, K, skip):
+    """Enough 128-blocks for the wide form: a last group of one block, three blocks per row, and pointers off the 16-byte
+    boundary, which keep the narrow one."""
+    x, w = synth.activations(1234, f"rot{K}", rows, K), synth.linear_weights(1234, f"rot{K}", K, 128, 4)
+    buf = torch.zeros(rows * K + skip, dtype=torch.float16, device="cuda")
+    buf[skip:] = dev(x).view(-1)
+    out = torch.empty((rows, K), dtype=torch.float16, device="cuda")
+    kernels.prefill_lin.had_r_128(buf[skip:], out, dev(w["suh"]), True, rows, K, False)
+    torch.cuda.synchronize()
+    assert (out.cpu().numpy().view(np.uint16) == oracle.had_r_128(x, w["suh"], True).view(np.uint16)).all()

@@ -170,6 +170,25 @@ __global__ void __launch_bounds__(256) k_silu_mul(const __half2* gate, const __h
     }
 }
 
+// The same for 16-byte aligned arrays, eight elements per thread and access.  Bound: the instructions of exp and of the six
+// fp16 roundings, next to HBM (6 bytes per element).  4096 rows of 17408: 147 -> 100 us with the reciprocal instruction, 421 rows 22.5 -> 16.4 us.
+__global__ void __launch_bounds__(256) k_silu_mul_wide(const uint4* gate, const uint4* up, uint4* out, long long octets, float limit)
+{
+    pdl_trigger();
+    pdl_wait();
+    for (long long i = (long long) blockIdx.x * 256 + threadIdx.x; i < octets; i += (long long) gridDim.x * 256) {
+        const uint4 g4 = gate[i], u4 = up[i];
+        const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, uw[4] = {u4.x, u4.y, u4.z, u4.w};
+        uint32_t ow[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const __half2 g = *reinterpret_cast<const __half2*>(&gw[j]), u = *reinterpret_cast<const __half2*>(&uw[j]);
+            ow[j] = dq::pack_half2(silu_mul_one(__low2half(g), __low2half(u), limit), silu_mul_one(__high2half(g), __high2half(u), limit));
+        }
+        out[i] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+    }
+}
+
 // The same over the first *n_rows rows of `row_pairs` half pairs each (row count known on the device only).
 __global__ void __launch_bounds__(256) k_silu_mul_rows(const __half2* gate, const __half2* up, __half2* out,
                                                        const int* __restrict__ n_rows, int max_rows, int row_pairs, float limit)
@@ -425,6 +444,14 @@ extern "C" int berth_ops_silu_mul(const void* gate, const void* up, void* out, i
         if (!gate || !up || !out) throw std::runtime_error("silu_mul: null device pointer");
         if (numel < 2 || (numel & 1)) throw std::runtime_error("silu_mul: numel must be positive and even");
         long long pairs = numel / 2;
+        const bool aligned = ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+        if (aligned && numel % 8 == 0 && numel >= 148LL * 8 * 256 * 2) {   // below, a thread's single pair spreads the work wider
+            const int wide = int(std::min<long long>((numel / 8 + 255) / 256, 148LL * 8));
+            launch_pdl(k_silu_mul_wide, dim3(wide), dim3(256), 0, (cudaStream_t) stream, "silu_mul launch", (const uint4*) gate, (const uint4*) up,
+                       (uint4*) out, (long long) (numel / 8), act_limit);
+            st.launch = "k_silu_mul_wide block=256 grid=" + std::to_string(wide);
+            return;
+        }
         int grid = int(std::min<long long>((pairs + 255) / 256, 148LL * 8));
         launch_pdl(k_silu_mul, dim3(grid), dim3(256), 0, (cudaStream_t) stream, "silu_mul launch", (const __half2*) gate,
                    (const __half2*) up, (__half2*) out, pairs, act_limit);

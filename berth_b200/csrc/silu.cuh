@@ -26,6 +26,17 @@ __device__ __forceinline__ float exp_f32_det(float x)
     return __fmul_rn(p, __int_as_float((int(n) + 127) << 23));
 }
 
+// 1/d to within a unit in the last fp32 place, for a d >= 1 that is an fp16 value: rounded to fp16 it equals the rounding of
+// the IEEE quotient.  A midpoint m of two fp16 values in (1/2, 1) is M / 2^12 (in lower binades the same, scaled) and
+// d is D / 2^10 times a power of two, so m d = 1 is impossible off the powers of two and |1 - m d| >= 2^-22: no midpoint
+// lies within 2^-22 of 1/d, and the instruction is off by at most 2^-23.  The IEEE division was a third of this function.
+__device__ __forceinline__ float rcp_of_half(float d)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return r;
+}
+
 // e = h(exp(-g)); d = h(1+e); r = h(1/d); s = h(g*r); out = h(s*u): every step rounded to fp16,
 // which reproduces berth's silu.out.bin fixture bit for bit.
 __device__ __forceinline__ __half silu_mul_one(__half g, __half u, float limit)
@@ -33,7 +44,7 @@ __device__ __forceinline__ __half silu_mul_one(__half g, __half u, float limit)
     const float gf = __half2float(g);
     __half e = (gf != gf) ? __ushort_as_half(0x7e00) : __float2half_rn(exp_f32_det(-gf));
     __half d = __float2half_rn(__fadd_rn(1.0f, __half2float(e)));
-    __half r = __float2half_rn(__fdiv_rn(1.0f, __half2float(d)));
+    __half r = __float2half_rn(rcp_of_half(__half2float(d)));
     __half s = __float2half_rn(__fmul_rn(gf, __half2float(r)));
     __half o = __float2half_rn(__fmul_rn(__half2float(s), __half2float(u)));
     if (limit != 0.0f) {

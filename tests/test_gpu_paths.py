@@ -108,3 +108,19 @@ def test_rotation_of_many_rows_bit_exact(oracle, rows, K, skip):
     kernels.prefill_lin.had_r_128(buf[skip:], out, dev(w["suh"]), True, rows, K, False)
     torch.cuda.synchronize()
     assert (out.cpu().numpy().view(np.uint16) == oracle.had_r_128(x, w["suh"], True).view(np.uint16)).all()
+
+
+@pytest.mark.parametrize("n,limit,skip", [(65536, 0.0, 0), (65536 * 16, 0.0, 0), (65536 * 16, 3.5, 0), (65536 * 16 + 2, 0.0, 0), (65536 * 16, 0.0, 2)])
+def test_silu_mul_every_gate_value_bit_exact(oracle, n, limit, skip):
+    """All 65536 fp16 patterns as gates (NaN and infinities among them), in the wide and the narrow form."""
+    gate = np.resize(np.arange(65536, dtype=np.uint16), n).view(np.float16)
+    up = synth.activations(1234, "silu.u", 1, n)[0]
+    g, u = (torch.zeros(n + skip, dtype=torch.float16, device="cuda") for _ in range(2))
+    g[skip:], u[skip:] = dev(gate), dev(up)
+    out = torch.empty(n, dtype=torch.float16, device="cuda")
+    kernels.ops.silu_mul(g[skip:], u[skip:], out, n, limit)
+    torch.cuda.synchronize()
+    got, exp = out.cpu().numpy(), oracle.silu_mul(gate, up, limit)
+    nan = np.isnan(exp)
+    assert (np.isnan(got) == nan).all()
+    assert (got.view(np.uint16)[~nan] == exp.view(np.uint16)[~nan]).all()

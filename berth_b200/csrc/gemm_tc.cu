@@ -514,6 +514,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
     if (team >= 0) {
         const int quarter = warp & 3;
         const int n = quarter * 32 + lane;
+        pdl_wait();   // svh may be the output of a kernel that is still running (the rotation before this launch triggers at its start)
         const float scale = __half2float(p.svh[size_t(z) * p.n + band * BN + n]);
         mbar_wait_parked(acc_full, 0, p.status, team == 0 ? 1000 : 100);
         tc_fence_after();

@@ -5,7 +5,7 @@ import pytest
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-from berth_b200 import kernels, moe, synth   # noqa: E402
+from berth_b200 import Codebook, OutDtype, kernels, moe, synth   # noqa: E402
 from tests.gpu_util import assert_close, dev, run_linear   # noqa: E402
 
 
@@ -124,3 +124,35 @@ def test_silu_mul_every_gate_value_bit_exact(oracle, n, limit, skip):
     nan = np.isnan(exp)
     assert (np.isnan(got) == nan).all()
     assert (got.view(np.uint16)[~nan] == exp.view(np.uint16)[~nan]).all()
+
+
+def _written_by_a_slow_kernel(seed, n):
+    """A buffer of n halves and a call that fills it on the stream with one row of RMSNorm: one block, which lets its successor
+    start at once and writes the end of the row last."""
+    x, wn = dev(synth.activations(seed, "slow.x", 1, n).astype(np.float32)), torch.zeros(n, dtype=torch.float16, device="cuda")
+    y = torch.zeros(n, dtype=torch.float16, device="cuda")
+    return y, lambda: kernels.ops.rms_norm(x, wn, y, 1, n, 1e-6, 1.0, 1.0, False)
+
+
+@pytest.mark.parametrize("m,K,N,bits,cb,kernel", [(1, 1024, 256, 4, 2, "k_exl3_gemv_i8"), (3, 1024, 256, 4, 2, "k_exl3_gemv_i8"), (8, 1024, 256, 4, 0, "k_exl3_gemv<"),
+                                                  (20, 2048, 5120, 4, 2, "splitk"), (40, 1024, 256, 4, 2, "x1x"), (40, 128, 512, 4, 2, "grid=4x1 "),
+                                                  (300, 1024, 256, 5, 1, "k_exl3_gemm_tc")])
+def test_output_scales_written_by_the_preceding_kernel(m, K, N, bits, cb, kernel):
+    """svh is touched only after the predecessor ended, on every path: it may be the preceding kernel's output."""
+    w = synth.linear_weights(1234, f"svh{K}x{N}", K, N, bits)
+    x, td, sd = dev(synth.activations(1234, f"svh.x{m}", m, K)), dev(w["trellis"]), dev(w["suh"])
+    slow, write = _written_by_a_slow_kernel(1234, 65536)
+    svh = slow[-N:]
+    c, ah = torch.empty((m, N), dtype=torch.float32, device="cuda"), torch.empty((m, K), dtype=torch.float16, device="cuda")
+    linear = lambda: kernels.exl3_linear(x, td, c, sd, ah, svh, m, K, N, bits, Codebook(cb), OutDtype.F32)
+    write()
+    torch.cuda.synchronize()
+    linear()
+    ref = c.cpu().numpy()
+    assert kernel in kernels.last_launch()
+    for _ in range(8):
+        slow.zero_()
+        torch.cuda.synchronize()
+        write()
+        linear()
+        assert (c.cpu().numpy().view(np.uint32) == ref.view(np.uint32)).all()

@@ -73,6 +73,13 @@ struct TGeo {
     static constexpr int kEpilogueExtra = (32 * 129 + 2 * 128) * 4;
     static constexpr int kFree = 227 * 1024 - 1024 - SA * A_STAGE_BYTES - kEpilogueExtra - kBarrierBytes - 2048 /*static shared*/;
     static constexpr int ST = kFree / T_STAGE_BYTES < 4 ? 4 : (kFree / T_STAGE_BYTES > 16 ? 16 : kFree / T_STAGE_BYTES);
+    // A decode group waits only for its own stages, every fourth one, and TMA copies finish out of order: with fewer than
+    // 2 * SW trellis stages (seven at 8 bits) a group that is done with stage i - 4 could look for stage i while stage i - ST,
+    // another group's and in the same slot, is still on its way, and take the phase BEFORE that one for its own (a parity wait
+    // cannot tell them apart): it would decode what the slot held and release it a second time.  The group then waits for
+    // its weight stage first: the MMAs of stage i - 4 are done, so every stage up to i - 4 has arrived.  (From 2 * SW stages on
+    // the weight stage of i - 4 says as much: the MMAs of stage i - 8 were done when it was stored.)
+    static constexpr bool ORDERED = ST < 2 * SW;
     static constexpr int RINGS = SA * A_STAGE_BYTES + ST * T_STAGE_BYTES;
     static constexpr int DENSE_RINGS = RINGS > kSplitEpilogueBytes ? RINGS : kSplitEpilogueBytes;   // (the dense kernel's epilogue lies over them)
     static constexpr size_t SMEM = 1024 /*align slack*/ + size_t(DENSE_RINGS) + kBarrierBytes;
@@ -492,6 +499,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
         static_assert(SW == 4 && ST >= 4, "one weight stage per decode group");
         int st = g, pt = 0, pw = 0;
         for (int ks = g; ks < kstages; ks += 4) {
+            if (TG_::ORDERED && ks >= SW) mbar_wait_parked(empty_w + 8 * g, pw ^ 1, p.status, 40);
             mbar_wait_parked(full_t + 8 * st, pt, p.status, 40);
             decode_stage<BITS, CB>(t_ring + st * T_STAGE_BYTES, tmem_w + g * 32, quarter, lane, ks >= SW, empty_w + 8 * g, pw ^ 1, p.status);
             if (lane == 0) {
@@ -756,6 +764,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc_grouped(const __gr
         int st = g, pt = 0, pw = 0;
         const int total = my_items * kstages;
         for (int cnt = g; cnt < total; cnt += G) {
+            if (TG_::ORDERED && cnt >= G) mbar_wait_parked(empty_w + 8 * g, pw ^ 1, p.status, 40);
             mbar_wait_parked(full_t + 8 * st, pt, p.status, 40);
             decode_stage<BITS, CB>(t_ring + st * T_STAGE_BYTES, tmem_w + g * 32, quarter, lane, cnt >= G, empty_w + 8 * g, pw ^ 1, p.status);
             if (lane == 0) {
@@ -892,6 +901,7 @@ template <int BITS>
 struct SGeo {
     static constexpr int T_STAGE_BYTES = TGeo<BITS>::T_STAGE_BYTES;
     static constexpr int ST = (160 * 1024) / T_STAGE_BYTES > 24 ? 24 : (160 * 1024) / T_STAGE_BYTES;   // 24 stages up to 6 bpw, 20 at 8
+    static_assert(ST >= kSkSW + 4, "order of the stages' arrival (see TGeo::ORDERED): the MMAs of stage i - 12 are done when a group looks for stage i");
     static constexpr int kBars = 2 * kSkSA + 2 * kSkSW + 2 * ST + 4;
     static constexpr size_t SMEM = 1024 /*align slack*/ + size_t(kSkSA) * kSkAStageBytes + size_t(ST) * T_STAGE_BYTES +
                                    (kXchFloats + 2 * 128) * 4 + kBars * 8;

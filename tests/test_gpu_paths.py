@@ -156,3 +156,38 @@ def test_output_scales_written_by_the_preceding_kernel(m, K, N, bits, cb, kernel
         write()
         linear()
         assert (c.cpu().numpy().view(np.uint32) == ref.view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("m,K,N,cb", [(40, 5120, 256, 0), (33, 5120, 1024, 2), (200, 2048, 512, 1), (421, 1024, 384, 2)])
+def test_prefill_8_bits_many_stages(oracle, m, K, N, cb):
+    """8 bits: seven trellis stages for four decode groups, whose phases are told apart by waiting in the MMAs' order."""
+    w = synth.linear_weights(1234, f"b8{K}", K, N, 8)
+    x = synth.activations(1234, f"b8{K}.x", m, K)
+    exp = oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, 8, cb)
+    first = None
+    for _ in range(20):
+        c, _ = run_linear(x, w, 8, cb, True, prefill=True)
+        assert first is None or c.tobytes() == first.tobytes()
+        first = c
+    assert "k_exl3_gemm_tc" in kernels.prefill_lin.last_launch()
+    assert_close(first, exp, "8 bits")
+    assert kernels.device_status(torch.cuda.current_device()) == 0
+
+
+@pytest.mark.parametrize("H,inter", [(512, 1152), (2048, 256)])
+def test_moe_layer_8_bits_tensor_core_stage(oracle, H, inter):
+    """The same in the grouped kernel: a long K (four decode groups) and a short one (three groups, two epilogue teams)."""
+    E, k, T = 32, 8, 128
+    wts = synth.moe_layer_weights(1234, "moe8", H, inter, E, k, 8, 2, shared_inter=inter)
+    x = synth.activations(1234, "moe8.x", T, H)
+    layer = moe.MoeLayer(torch.device("cuda"), wts, T)
+    out = torch.full((T, H), float("nan"), dtype=torch.float32, device="cuda")
+    idx, w = torch.empty((T, k), dtype=torch.int32, device="cuda"), torch.empty((T, k), dtype=torch.float32, device="cuda")
+    for _ in range(10):
+        layer.forward(dev(x), out, idx, w)
+        torch.cuda.synchronize()
+    assert "k_exl3_gemm_tc_grouped" in moe.last_launch()
+    assert kernels.device_status(torch.cuda.current_device()) == 0
+    _, exp_idx, exp_w = oracle.moe_layer(wts, x)
+    assert (idx.cpu().numpy() == exp_idx).all()
+    assert_close(out.cpu().numpy(), oracle.moe_layer_f64(wts, x, exp_idx, exp_w), "8 bits")

@@ -17,7 +17,7 @@ __host__ __device__ inline int unit_owner(long long u, long long U, int G) { ret
 
 // Bits of the status word a bounded wait sets when it runs out: a weight stage never arrived / was never
 // released (TMA ring), a tensor-memory stage or accumulator was never handed over (integer tensor path).
-enum StatusBits : unsigned { kStFullTimeout = 1u, kStEmptyTimeout = 2u, kStTmemTimeout = 4u };
+enum StatusBits : unsigned { kStFullTimeout = 1u, kStEmptyTimeout = 2u, kStTmemTimeout = 4u, kStOverflow = 64u /*a problem table with more rows or problems than the launch was sized for*/ };
 
 
 constexpr int kMaxHetMatrices = 4;

@@ -263,6 +263,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
     const int bands = p.n >> 7, kblocks = p.k >> 7;
     const int bgroups = (bands + BU - 1) / BU;
     const int nprob = GROUPED ? min(max(__ldg(p.n_problems), 0), p.max_problems) : (p.n_stack > 1 ? p.n_stack : 1);
+    if (GROUPED && blockIdx.x == 0 && threadIdx.x == 0 && __ldg(p.n_problems) > p.max_problems) atomicOr(p.status, kStOverflow);
     const long long U = p.het ? (long long) p.het_bg[p.n_stack] * kblocks : (long long) nprob * bgroups * kblocks;
     // band group of the launch -> matrix and band group inside it
     auto split_bg = [&](int gbg, int& pi, int& lbg) {
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
     const int pre0 = pre < kPre0 ? pre : kPre0;
     constexpr uint32_t kStageTx = FUSED ? W_BYTES : STAGE_BYTES;
     auto issue_weights = [&](uint32_t dst, uint32_t bar) {
-        const int z = GROUPED ? load_problem(p.problems, pr_pi, p.n_matrices, TOK, p.max_rows).z : (p.het ? 0 : pr_pi);
+        const int z = GROUPED ? load_problem(p.problems, pr_pi, p.n_matrices, p.m, p.max_rows).z : (p.het ? 0 : pr_pi);
         tma_load_3d(dst, &maps.m[p.het ? pr_pi : 0], pr_lbg * (ROW_BYTES / 8), pr_kb * 8, z, bar);
     };
     auto next_unit = [&]() {
@@ -373,7 +374,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
                     const __half* suh = p.het ? p.het_suh[pi] : p.suh + size_t(pi) * p.k;
                     int src = t;
                     if constexpr (GROUPED) {
-                        const GemvProblem pr = load_problem(p.problems, pi, p.n_matrices, TOK, p.max_rows);
+                        const GemvProblem pr = load_problem(p.problems, pi, p.n_matrices, p.m, p.max_rows);
                         if (t >= pr.rows) continue;
                         suh = pr.z < p.z_half ? p.suh + size_t(pr.z) * p.k : p.suh_b + size_t(pr.z - p.z_half) * p.k;
                         const int r = pr.row0 + t - (pr.row0 >= p.row_half ? p.row_half : 0);
@@ -555,7 +556,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
             const Segment sg = segment_at(u, u0, u1, kblocks);
             int pi, lbg;
             split_bg(sg.bg, pi, lbg);
-            ProblemView pv = problem_view<GemvArgs, GROUPED>(p, pi, TOK);
+            // (a problem has at most p.m rows: what was rotated, and what a slab holds)
+            ProblemView pv = problem_view<GemvArgs, GROUPED>(p, pi, p.m);
+            if (GROUPED && et == 0 && p.problems[pi].rows > p.m) atomicOr(p.status, kStOverflow);
             if (p.het) {
                 pv.z = 0; pv.act = pi;
                 pv.svh = p.het_svh[pi]; pv.c = p.het_c[pi]; pv.ldc = p.het_n[pi];

@@ -1456,9 +1456,12 @@ extern "C" int berth_moe_p2p_experts(const berth_moe_weights* w, const void* x_l
         __half* xr = static_cast<__half*>(pr.p[rank]);
         RowSource in_place{};
         in_place.paired = up_behind_gate(w, NM);
-        if (world == 1 && T_local >= 1 && T_local <= 4) {   // (more ranks: how many rows arrive is known on the device only)
-            in_place.rows_per_problem = T_local;
-            in_place.most = std::min(T_local * top_k, NL) + (TS ? 1 : 0);
+        // the rows that arrive are those of send_tokens tokens, at most one per token in an expert; the shared expert's are TS
+        // (more ranks: how many rows arrive is known on the device only)
+        const int most_rows = std::max(send_tokens, TS);
+        if (world == 1 && most_rows >= 1 && most_rows <= 4) {
+            in_place.rows_per_problem = most_rows;
+            in_place.most = std::min(std::max(send_tokens, 0) * top_k, NL) + (TS ? 1 : 0);
         }
         launch_pdl(k_moe_scan, dim3(1), dim3(1024), 0, cs, "k_moe_scan launch", es.counts, es.offsets, es.problems, es.n_problems, NL, plan.chunk, TS,
                    in_place.paired ? max_rows : 0, NM, es.max_problems, max_rows, sc.status);

@@ -158,6 +158,45 @@ def test_output_scales_written_by_the_preceding_kernel(m, K, N, bits, cb, kernel
         assert (c.cpu().numpy().view(np.uint32) == ref.view(np.uint32)).all()
 
 
+@pytest.mark.parametrize("send,local", [(6, 1), (6, 2), (9, 3), (6, 0), (2, 4), (1, 3), (4, 4), (3, 1)])
+def test_peer_experts_of_more_sent_than_local_tokens(oracle, send, local):
+    """berth_moe_p2p_experts takes the tokens that were sent and those of the shared expert apart: one rank that is its own peer,
+    its "symmetric" buffers ordinary allocations.  The sent tokens' rows come back as the oracle's layer without a shared
+    expert, the shared rows as its difference to the layer with one."""
+    import ctypes as C
+    from berth_b200 import _lib
+    H, I, E, k, bits = 256, 128, 32, 4, 4
+    l, device = _lib.lib(), torch.device("cuda", torch.cuda.current_device())
+    wts = synth.moe_layer_weights(1234, "p2pn", H, I, E, k, bits, 2, shared_inter=I)
+    stages = moe.GpuStages(device, wts, E, max_rows=128, max_rows_per_expert=32)
+    assert stages.shared_is_stacked()
+    xh = synth.activations(1234, "p2pn.x", max(send, local), H)
+    x, max_rows = dev(xh), send * k + max(send, local) + 1
+    z = lambda n, dt=torch.uint8: torch.zeros(n, dtype=dt, device=device)
+    cnt, flags, recv, ret = z(E * 4), z(3 * 8 * 4), z(max_rows * H * 2), torch.full((send * k, H), float("nan"), dtype=torch.float16, device=device)
+    ptr = lambda t: (C.c_void_p * 1)(t.data_ptr())
+    send_ws, ws = z(l.berth_moe_p2p_send_workspace_bytes(send, E, k, 1)), z(l.berth_moe_p2p_experts_workspace_bytes(max_rows, E, H, I))
+    idx, w, inv = z(send * k, torch.int32), z(send * k, torch.float32), z(send * k, torch.int32)
+    ysh = torch.full((max(local, 1), H), float("nan"), dtype=torch.float16, device=device)
+    for epoch in (1, 2):
+        assert l.berth_moe_p2p_send(x.data_ptr(), send, stages.layer._keep["w_router"].data_ptr(), None, H, E, k, idx.data_ptr(), w.data_ptr(),
+                                    inv.data_ptr(), 0, 1, epoch, ptr(cnt), ptr(flags), ptr(recv), max_rows, send_ws.data_ptr(), send_ws.numel(), None) == 0
+        assert l.berth_moe_p2p_experts(C.byref(stages.layer.c), x.data_ptr(), local, ysh.data_ptr() if local else None, 0, 1, epoch, E, k, send,
+                                       ptr(cnt), ptr(flags), ptr(recv), ptr(ret), max_rows, send * k, 8, send_ws.data_ptr(), ws.data_ptr(),
+                                       ws.numel(), None) == 0, moe.last_error()
+    assert ("fused,grouped" in moe.last_launch()) == (max(send, local) <= 4)
+    out = stages.combine(ret, inv, w.view(send, k), None)
+    torch.cuda.synchronize()
+    assert kernels.device_status(device.index) == 0
+    alone = dict(wts, shared_inter=0)
+    _, exp_idx, exp_w = oracle.moe_layer(alone, xh)
+    assert (idx.view(send, k).cpu().numpy() == exp_idx[:send]).all()
+    routed = oracle.moe_layer_f64(alone, xh, exp_idx, exp_w)
+    assert_close(out.cpu().numpy(), routed[:send], "routed")
+    if local:
+        assert_close(ysh.cpu().numpy(), (oracle.moe_layer_f64(wts, xh, exp_idx, exp_w) - routed)[:local], "shared")
+
+
 @pytest.mark.parametrize("m,K,N,cb", [(40, 5120, 256, 0), (33, 5120, 1024, 2), (200, 2048, 512, 1), (421, 1024, 384, 2)])
 def test_prefill_8_bits_many_stages(oracle, m, K, N, cb):
     """8 bits: seven trellis stages for four decode groups, whose phases are told apart by waiting in the MMAs' order."""

@@ -96,7 +96,7 @@ struct GemmArgs {
     const int* n_problems;
     int max_problems, n_matrices;
     int split;          // dense launch: CTAs of a cluster along z that share a tile's K (1 = the tile is one CTA's)
-    int defer_weights;  // no weight fetch before griddepcontrol.wait (berth_exl3_weights_streamed)
+    int defer_weights;  // no L2 prefetch of the weights before griddepcontrol.wait either (berth_exl3_weights_streamed)
     int epi2;   // grouped launch with 128-row problems and a short K: two epilogue teams and three decode groups (see the kernel)
 };
 
@@ -164,6 +164,11 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
                  : "memory");
+}
+// The box into L2 only, where later writes to that memory still reach it.
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int x, int y, int z)
+{
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(x), "r"(y), "r"(z) : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -444,11 +449,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
                 tma_load_3d(smem_u32(t_ring + st * T_STAGE_BYTES), &tmap_t, band * (TROW_BYTES / 8), (k0 + ks) * 4, z, full_t + 8 * st);
                 if (++st == ST) { st = 0; pt ^= 1; }
             };
-            // the weights do not depend on the rotation kernel: the first lap of the ring is requested before the wait for it
+            // The first lap of the ring is asked into L2 while the rotation still runs, and read after the wait: a kernel before
+            // it may have written the weights, which a copy into shared memory ahead of the wait would miss.  (One layer,
+            // 40 / 421 rows: 222.8 / 494.8 us, with that copy 221.2 / 492.9, without the hint 229.3 / 493.0.)
             const int pre = min(kstages, ST);
-            if (p.defer_weights) pdl_wait();
-            for (int ks = 0; ks < pre; ++ks) load_trellis(ks);
+            if (!p.defer_weights)
+                for (int ks = 0; ks < pre; ++ks) tma_prefetch_3d(&tmap_t, band * (TROW_BYTES / 8), (k0 + ks) * 4, z);
             pdl_wait();
+            for (int ks = 0; ks < pre; ++ks) load_trellis(ks);
             for (int ks = 0; ks < kstages; ++ks) {
                 if (ks >= ST) {
                     mbar_wait_parked(empty_t + 8 * st, pt ^ 1, p.status, 100);

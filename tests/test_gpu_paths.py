@@ -158,6 +158,34 @@ def test_output_scales_written_by_the_preceding_kernel(m, K, N, bits, cb, kernel
         assert (c.cpu().numpy().view(np.uint32) == ref.view(np.uint32)).all()
 
 
+@pytest.mark.parametrize("m,K,N,bits,cb,guard", [(1, 1024, 256, 4, 2, True), (3, 1024, 256, 4, 2, True), (8, 1024, 256, 4, 0, True), (20, 2048, 5120, 4, 2, True),
+                                                 (40, 1024, 256, 4, 2, False), (40, 1024, 256, 4, 2, True), (40, 128, 512, 4, 2, False),
+                                                 (300, 1024, 256, 5, 1, False), (300, 512, 4096, 3, 2, False)])
+def test_weights_written_by_the_preceding_kernel(m, K, N, bits, cb, guard):
+    """The trellis as the output of the kernel that directly precedes the linear: above 32 rows at any time, on the decode
+    kernels with berth_exl3_weights_streamed(1)."""
+    w = synth.linear_weights(1234, f"trw{K}x{N}", K, N, bits)
+    x, sd, vd = dev(synth.activations(1234, f"trw.x{m}", m, K)), dev(w["suh"]), dev(w["svh"])
+    trellis, write = _written_by_a_slow_kernel(1234, K * N * bits // 16)
+    c, ah = torch.empty((m, N), dtype=torch.float32, device="cuda"), torch.empty((m, K), dtype=torch.float16, device="cuda")
+    linear = lambda: kernels.exl3_linear(x, trellis, c, sd, ah, vd, m, K, N, bits, Codebook(cb), OutDtype.F32)
+    write()
+    torch.cuda.synchronize()
+    linear()
+    ref = c.cpu().numpy()
+    assert np.isfinite(ref).all()
+    assert kernels.weights_streamed(guard) is False
+    try:
+        for _ in range(8):
+            trellis.zero_()
+            torch.cuda.synchronize()
+            write()
+            linear()
+            assert (c.cpu().numpy().view(np.uint32) == ref.view(np.uint32)).all()
+    finally:
+        kernels.weights_streamed(False)
+
+
 @pytest.mark.parametrize("send,local", [(6, 1), (6, 2), (9, 3), (6, 0), (2, 4), (1, 3), (4, 4), (3, 1)])
 def test_peer_experts_of_more_sent_than_local_tokens(oracle, send, local):
     """berth_moe_p2p_experts takes the tokens that were sent and those of the shared expert apart: one rank that is its own peer,

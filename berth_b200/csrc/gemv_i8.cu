@@ -15,7 +15,7 @@
 // enter as 16-bit block fixed point: per (row, 128 rotated inputs) one fp32 scale = max|a| / 32512 and
 // v = rint(a / scale), split into two signed 8-bit limbs v = 256 hi + lo.  The limbs of a row are two
 // of the N columns of the MMA; the s32 accumulation is exact and is folded into an fp32 accumulator
-// once per 128 inputs: acc += 2 scale * (128 hi_sum + lo_sum / 2).  The constant term uses the same
+// once per 128 inputs: acc += scale * (256 hi_sum + lo_sum).  The constant term uses the same
 // quantised values (block sums = scale * sum v), so the result is exactly the product with the
 // quantised activations up to fp32 rounding.  The fp32 rotated values are quantised, not their fp16
 // roundings (which the caller's buffer receives): the step is 2^-15 of the block maximum, a rounding error of
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
                     int isum;
                     const float scale = quantise_block(rot, lane, area + size_t(j) * ftile + t * 32, 2 * flbo, flbo, isum);
                     if (lane == 0) {
-                        fscales[j * 8 + t] = 2.0f * scale;
+                        fscales[j * 8 + t] = scale;
                         fscales[j * 8 + 4 + t] = __fmul_rn(scale, __int2float_rn(isum));
                     }
                     if (lbg == 0 && !GROUPED) {   // band group 0 of a matrix meets every 128-block exactly once: the caller's copy
@@ -611,10 +611,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
                     sxp[t] = __fadd_rn(sxp[t], bs[t]);
 #pragma unroll
                     for (int b = 0; b < BU; ++b)
-                        // half of 256 hi + lo, against twice the scale: the whole can pass 2^31 (a block whose rotated values are all
-                        // alike, as those of a one-hot input are), the half stays below 128 * 1020 * 127 * 128 + 2^23 < 2^31; the bit
-                        // that falls off is below the conversion's own rounding
-                        acc[b][t] = __fmaf_rn(sc[t], __int2float_rn(r[b][2 * t] * 128 + (r[b][2 * t + 1] >> 1)), acc[b][t]);
+                        // 256 hi + lo rounded once to fp32; as an integer it can pass 2^31 (a block whose rotated values are all alike, as
+                        // those of a one-hot input are), while each sum is below 128 * 1020 * 128 < 2^24 and converts exactly
+                        acc[b][t] = __fmaf_rn(sc[t], __fmaf_rn(256.0f, __int2float_rn(r[b][2 * t]), __int2float_rn(r[b][2 * t + 1])), acc[b][t]);
                 }
             }
             // ---- the segment's sums: thread et owns column et of every band
@@ -728,7 +727,7 @@ __global__ void __launch_bounds__(128) k_rotate_in_i8(const __half* __restrict__
         if (lane == 0) {
             float* tail = reinterpret_cast<float*>(limbs + size_t(b) * record + size_t(16) * nb * 256);   // 16 scales, then 16 block sums
             const float bsum = __fmul_rn(scale, __int2float_rn(isum));
-            tail[row] = 2.0f * scale;
+            tail[row] = scale;
             tail[16 + row] = bsum;
             blocksum[size_t(row) * kblocks + b] = bsum;
         }

@@ -21,6 +21,30 @@ def test_integer_path_one_hot_blocks(oracle):
     assert_close(c, oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, cb), "one-hot blocks")
 
 
+@pytest.mark.parametrize("m,bits", [(1, 4), (1, 5), (4, 4), (4, 5)])
+def test_integer_path_sums_are_rounded_not_cut(oracle, m, bits):
+    """A row that rotates to two non-zero values, quantised to 32512 and 13, so that the integer sum of a column is known:
+    32512 u1 + 13 u2 (u the weights' byte sums).  The first output of a band adds its 128 columns: rounding errors of a sum (half a
+    unit) average out over 96 bands, to about 12 / sqrt(96) units by the fp32 roundings behind them, a low bit that is always
+    dropped (half a unit of every column) does not: 64."""
+    f, N, i0, i1 = np.float32, 128 * 96, 5, 77
+    w = synth.linear_weights(1234, f"round{bits}", 128, N, bits)
+    sign = np.array([[(-1) ** bin(i & j).count("1") for j in range(128)] for i in (i0, i1)])
+    same = sign[0] == sign[1]
+    x = np.where(same, 1301, 1413) / 128 * sign[0]                       # times suh: (32512 s0 + 13 s1) / 128
+    w["suh"], w["svh"] = np.where(same, 25, 23).astype(np.float16), np.ones(N, np.float16)
+    u = np.rint((oracle.reconstruct(w["trellis"], 128, N, bits, 2).view(np.float16).reshape(128, N).astype(np.float64) + 10.3828125) / 0.00676727294921875) - 1024
+    total = 32512 * u[i0] + 13 * u[i1]
+    scale = f(f(32512) * f(0.088388347648)) * f(1 / 32512)
+    constant = f(f(-3.453125) * f(scale * f(32525)))
+    exp = (0.00676727294921875 * np.float64(scale) * total + np.float64(constant)).reshape(96, 128).sum(1) * 0.088388347648
+    c, _ = run_linear(np.tile(x, (m, 1)).astype(np.float16), w, bits, 2, True)
+    assert "k_exl3_gemv_i8" in kernels.last_launch()
+    for row in c:
+        units = (row[::128] - exp) / (0.00676727294921875 * np.float64(scale) * 0.088388347648)
+        assert abs(units.mean()) < 8 and np.abs(units).max() < 200, (units.mean(), np.abs(units).max())
+
+
 @pytest.mark.parametrize("bits", [3, 4, 5, 6])
 @pytest.mark.parametrize("K,N", [(128, 128 * 301), (384, 256 * 160 + 128)])
 def test_integer_path_several_band_groups_per_cta(oracle, K, N, bits):

@@ -808,8 +808,32 @@ size_t launch_bits(int k_bits, int nb, bool fused, const void* const* t, int nm,
 
 }  // namespace
 
-// Whether launch_gemv sends a dense MUL1 linear here: the rotation fits the kernel and the scratch suffices (where it does
-// not, the fp16-path kernel still serves the shape).
+// Two to four rows of one matrix: whether this kernel is at least as fast as k_exl3_gemv with its rotation (from three rows on a
+// launch of its own) and finishing launches.  Both were timed for 111 matrices from 128 x 512 to 17408 x 17408 at 2, 3, 4, 5, 6
+// and 8 bits, weights out of cache.  This kernel rotates rows * (128-blocks of a CTA) blocks before its first MMA and saves launches; its
+// decode is ahead where a unit is one band (5 bits and more) and level below.  So, with `units` = units of a CTA:
+//  - up to 4 bits: where a CTA holds whole band groups and meets few 128-blocks (128 x 6144, two rows: 4.0 against 5.4 us), where K
+//    is so short that the launches are everything (kblocks <= 4), and at 4 bits for a vocabulary's width (5120 x 151552,
+//    two rows: 160 against 166 us).  Elsewhere it loses: 5120 x 1024, four rows: 14.2 against 11.3 us;
+//  - from 5 bits on: whole band groups (5120 x 151552 at 6 bits, three rows: 209 against 254 us; with four rows from one and a half or two of them a CTA),
+//    few bands (5120 x 1024, four rows: 9.3 against 11.6), three rows of all but short matrices (5120 x 6144: 17.1 against 20.0),
+//    four while the rotation is short; two rows only where the other kernel cannot rotate in the launch itself (more than 26
+//    units; 5120 x 6144: 17.6 against 15.5).
+// No point of the sweep is more than 2.5 % slower here than there, and five of 920 are more than 1 %.
+static bool few_rows_pay(int rows, int k_bits, long long units, int kblocks, bool few_bands)
+{
+    const bool whole = units >= kblocks;
+    if (k_bits <= 4)
+        return (whole && (kblocks <= (rows == 2 ? 16 : 2) || (k_bits == 4 && rows < 4 && units >= 4LL * kblocks))) ||
+               (kblocks <= 4 && (few_bands || units >= 4LL * kblocks));
+    if (whole) return rows < 4 || kblocks <= 2 || units >= 2LL * kblocks || (kblocks <= 16 && 2 * units >= 3LL * kblocks);
+    if (few_bands) return true;
+    if (rows == 2) return units > 26 && units <= 50;
+    return rows == 3 ? kblocks >= 8 : (kblocks >= 16 || 2 * units < kblocks) && units < 10;
+}
+
+// Whether launch_gemv sends a dense MUL1 linear here: it pays, the rotation fits the kernel and the scratch suffices (where it
+// does not, the fp16-path kernel still serves the shape).
 bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc)
 {
     if (size_m < 1 || size_m > 4 || size_k % 128 != 0 || size_n % 128 != 0 || k_bits < 1 || k_bits > 8) return false;
@@ -817,7 +841,10 @@ bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, con
     const int bands = size_n / 128, kblocks = size_k / 128, bgroups = (bands + bu - 1) / bu;
     const long long units = (long long) bgroups * kblocks;
     const int grid = int(std::min<long long>(std::min<long long>(sms, units), (long long) bgroups * 16));
-    if (grid < 1 || std::min<long long>((units + grid - 1) / grid, kblocks) > fused_max_units(k_bits, size_m)) return false;
+    if (grid < 1) return false;
+    const long long units_per_cta = (units + grid - 1) / grid;
+    if (std::min<long long>(units_per_cta, kblocks) > fused_max_units(k_bits, size_m)) return false;
+    if (size_m > 1 && !few_rows_pay(size_m, k_bits, units_per_cta, kblocks, grid < sms)) return false;
     return size_t(bgroups) <= sc.counter_words && size_t(size_m) * kblocks <= sc.blocksum_floats &&
            size_t(kblocks) * (size_t(16) * 256 + 128) <= sc.afrag_bytes &&
            size_t(grid) * 2 * (size_t(size_m) * bu * 128 + 32) * sizeof(float) <= sc.slab_bytes;

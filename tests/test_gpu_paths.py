@@ -56,13 +56,16 @@ def test_integer_path_several_band_groups_per_cta(oracle, K, N, bits):
     assert_close(c, oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, 2), "wide")
     assert kernels.device_status(torch.cuda.current_device()) == 0
 
-@pytest.mark.parametrize("m", [2, 3, 4])
-@pytest.mark.parametrize("K,N,bits", [(5120, 1024, 4), (2176, 3072, 5), (128, 128 * 301, 6), (1152, 640, 3)])
-def test_integer_path_two_to_four_rows(oracle, m, K, N, bits):
+@pytest.mark.parametrize("m,K,N,bits,here", [(m, K, N, bits, m in where) for K, N, bits, where in [
+    (5120, 1024, 4, ()), (5120, 1024, 5, (2, 3, 4)), (2176, 3072, 5, (3, 4)), (1024, 6144, 5, (3, 4)), (1024, 8192, 6, (3,)), (896, 8192, 6, ()), (128, 128 * 301, 6, (2, 3, 4)),
+    (384, 128 * 301, 5, (2, 3, 4)), (384, 128 * 200, 6, (2, 3, 4)), (2048, 128 * 200, 6, (2, 3)), (1152, 640, 3, ()), (384, 640, 3, (2, 3, 4)), (256, 128 * 301, 4, (2, 3, 4)),
+    (2048, 128 * 301, 4, (2,)), (2176, 128 * 301, 4, ()), (3584, 128 * 130, 5, (3,)), (1024, 128 * 240, 5, (2, 3, 4)), (2048, 128 * 100, 8, (3,))] for m in (2, 3, 4)])
+def test_integer_path_two_to_four_rows(oracle, m, K, N, bits, here):
+    """Both sides of each line of the rule that picks the kernel."""
     w = synth.linear_weights(1234, f"few{K}{bits}", K, N, bits)
     x = synth.activations(1234, f"few{K}.x{m}", m, K)
     c, ah = run_linear(x, w, bits, 2, False)
-    assert "k_exl3_gemv_i8" in kernels.last_launch()
+    assert ("k_exl3_gemv_i8" in kernels.last_launch()) == here and ("fused" in kernels.last_launch() or not here)
     assert_close(c, oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, 2), "few rows")
     assert (ah == oracle.had_r_128(x, w["suh"], True).view(np.uint16)).all()
 
@@ -158,7 +161,7 @@ def _written_by_a_slow_kernel(seed, n):
     return y, lambda: kernels.ops.rms_norm(x, wn, y, 1, n, 1e-6, 1.0, 1.0, False)
 
 
-@pytest.mark.parametrize("m,K,N,bits,cb,kernel", [(1, 1024, 256, 4, 2, "k_exl3_gemv_i8"), (3, 1024, 256, 4, 2, "k_exl3_gemv_i8"), (8, 1024, 256, 4, 0, "k_exl3_gemv<"),
+@pytest.mark.parametrize("m,K,N,bits,cb,kernel", [(1, 1024, 256, 4, 2, "k_exl3_gemv_i8"), (3, 1024, 256, 5, 2, "k_exl3_gemv_i8"), (8, 1024, 256, 4, 0, "k_exl3_gemv<"),
                                                   (20, 2048, 5120, 4, 2, "splitk"), (40, 1024, 256, 4, 2, "x1x"), (40, 128, 512, 4, 2, "grid=4x1 "),
                                                   (300, 1024, 256, 5, 1, "k_exl3_gemm_tc")])
 def test_output_scales_written_by_the_preceding_kernel(m, K, N, bits, cb, kernel):

@@ -808,6 +808,16 @@ size_t launch_bits(int k_bits, int nb, bool fused, const void* const* t, int nm,
 
 }  // namespace
 
+// Launches over several matrices: whether a CTA rotates its own tiles, or one k_rotate_in_i8 per matrix does before.  Twenty warps
+// rotate a block each in about 1.7 us; with two or four rows the replicated words of a warp fall on half as many banks as
+// with one or three (the limb rows are 64 * rows bytes apart), and above 80 blocks a CTA the launches cost less: two rows of a
+// 5120 x 13824 pair at 5 bits (118 blocks) 55.7 against 50.1 us, four rows of a 3584 x 10752 pair (128) 39.4 against 34.7; three rows of
+// a 5120 x 17408 pair at 4 bits (111) 50.4 here and 52.1 with them.
+static bool stack_rotates_in_kernel(int k_bits, int rows, long long tiles)
+{
+    return tiles <= fused_max_units(k_bits, rows) && (rows % 2 != 0 || rows * tiles <= 80);
+}
+
 // Two to four rows of one matrix: whether this kernel is at least as fast as k_exl3_gemv with its rotation (from three rows on a
 // launch of its own) and finishing launches.  Both were timed for 111 matrices from 128 x 512 to 17408 x 17408 at 2, 3, 4, 5, 6
 // and 8 bits, weights out of cache.  This kernel rotates rows * (128-blocks of a CTA) blocks before its first MMA and saves launches; its
@@ -882,7 +892,7 @@ std::string launch_gemv_i8(const void* a, const void* trellis, void* c, const vo
     // matrix never more than the row has 128-blocks.
     long long tiles_per_cta = (units + grid - 1) / grid;
     if (n_stack == 1) tiles_per_cta = std::min<long long>(tiles_per_cta, kblocks);
-    const bool fused = nb == 1 && tiles_per_cta <= fused_max_units(k_bits, size_m);
+    const bool fused = nb == 1 && (n_stack > 1 ? stack_rotates_in_kernel(k_bits, size_m, tiles_per_cta) : tiles_per_cta <= fused_max_units(k_bits, size_m));
     const int rot_total = size_m * kblocks;
     if (!fused)
         for (int i = 0; i < n_stack; ++i)
@@ -961,7 +971,7 @@ std::string launch_gemv_i8_multi(const void* a, const void* const* trellis, void
     if (grid < 1) throw std::runtime_error("exl3 gemv: split-K scratch is too small for this shape");
     if (size_t(total_bg) > sc.counter_words) throw std::runtime_error("exl3 gemv: band groups exceed the counters of the scratch");
     const long long units_per_cta = (units + grid - 1) / grid;
-    const bool fused = nb == 1 && units_per_cta <= fused_max_units(k_bits, size_m);
+    const bool fused = nb == 1 && stack_rotates_in_kernel(k_bits, size_m, units_per_cta);
     const int rot_total = size_m * kblocks;
     if (!fused)
         for (int i = 0; i < n_matrices; ++i)

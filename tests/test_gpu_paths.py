@@ -69,6 +69,20 @@ def test_integer_path_two_to_four_rows(oracle, m, K, N, bits, here):
     assert_close(c, oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, 2), "few rows")
     assert (ah == oracle.had_r_128(x, w["suh"], True).view(np.uint16)).all()
 
+@pytest.mark.parametrize("m,N,inside", [(2, 128 * 720, True), (2, 128 * 760, False), (3, 128 * 720, True), (4, 128 * 360, True), (4, 128 * 380, False)])
+def test_stack_rotation_inside_or_before(oracle, m, N, inside):
+    """78 and 84 blocks a CTA of two rows, 117 of three, 80 and 84 of four: rotated in the launch or by launches before it."""
+    K, bits, ns = 512, 5, 2
+    ws = [synth.linear_weights(1234, f"stk{N}.{i}", K, N, bits) for i in range(ns)]
+    x = synth.activations(1234, f"stk.x{m}", m, K)
+    tr, su, sv = (torch.stack([dev(w[k]) for w in ws]) for k in ("trellis", "suh", "svh"))
+    c, ah = torch.empty((ns, m, N), dtype=torch.float32, device="cuda"), torch.empty((ns, m, K), dtype=torch.float16, device="cuda")
+    kernels.exl3_linear_stack(dev(x), tr, c, su, ah, sv, ns, m, K, N, bits, Codebook(2), OutDtype.F32)
+    torch.cuda.synchronize()
+    assert ("fused" in kernels.last_launch()) == inside and "k_exl3_gemv_i8" in kernels.last_launch()
+    for i, w in enumerate(ws):
+        assert_close(c[i].cpu().numpy(), oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, 2), "stack")
+
 @pytest.mark.parametrize("T", [1, 2, 3, 4, 5, 9])
 @pytest.mark.parametrize("bits,inter,shared,E", [(4, 128, 128, 32), (3, 384, 384, 64), (5, 256, 0, 32)])
 def test_moe_layer_few_tokens_vs_oracle(oracle, T, bits, inter, shared, E):

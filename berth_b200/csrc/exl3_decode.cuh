@@ -127,6 +127,12 @@ __device__ __forceinline__ void states_aligned(uint32_t a0, uint32_t a1, uint32_
     }
 }
 
+// The share for the kernels that store the weights to tensor memory: all masks on the FMA-heavy pipe beside 3INST and MCG, and
+// for MUL1 up to 3 bits, two of them above (MoE layer of 1024 tokens at 3 bits, 128 experts of 512: 314 -> 305 us; 32 rows of
+// 5120 x 17408 at 2 bits: 39.1 -> 35.7 us; at 5 bits all of them cost 0.4 %).
+template <int BITS, int CB>
+__host__ __device__ constexpr int tc_window_heavy() { return CB != 2 || BITS <= 3 ? 8 : 2; }
+
 // Loads the lane's words from a tile (global or shared pointer to its 8*BITS raw words), with
 // the tail-biting wrap, and returns the eight states.
 template <int BITS, int HEAVY = 0>
@@ -209,9 +215,11 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
 template <int BITS, int CB>
 __device__ __forceinline__ void tile_states(const uint32_t* tile, int lane, int lane1, uint32_t (&s)[8])
 {
-    // the codebooks whose arithmetic leans on the ALU pipe take their half-word selections on the FMA-heavy pipe
+    // the codebooks whose arithmetic leans on the ALU pipe take their half-word selections on the FMA-heavy pipe; at 8 bits,
+    // where two of eight windows are a permute already, it is the other way round (8 rows of 5120 x 17408: 3INST 36.9 -> 34.0 us,
+    // MCG 35.9 -> 33.9, MUL1 37.9 -> 36.2)
     if constexpr (BITS == 4) states_4bit<(CB != 2) ? 6 : 0>(tile[lane], tile[lane1], s);
-    else lane_states<BITS, (CB != 2) ? 8 : 2>(tile, lane, s);
+    else lane_states<BITS, (CB != 2) ? (BITS == 8 ? 0 : 8) : (BITS == 8 ? 8 : 2)>(tile, lane, s);
 }
 
 // Duplicated activation pairs for the lo/hi-as-k-slots scheme: from b0 = (x[2q], x[2q+1]) and

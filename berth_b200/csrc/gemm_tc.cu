@@ -367,7 +367,7 @@ __device__ __forceinline__ void decode_stage(const unsigned char* tstage, uint32
             uint32_t s[8];
             const uint32_t* tile = trow + (2 * quarter + t) * NW;
             if constexpr (BITS == 4) dq::states_4bit<(CB != 2) ? 6 : 0>(tile[lane], tile[(lane + 1) & 31], s);
-            else dq::lane_states<BITS, (CB != 2) ? 8 : 2>(tile, lane, s);
+            else dq::lane_states<BITS, dq::tc_window_heavy<BITS, CB>()>(tile, lane, s);
             dq::decode_frag<CB>(s, w[t]);
         }
         if (krow == 0 && wait_w) {   // the MMAs that read this weight stage are done
@@ -857,7 +857,7 @@ __device__ __forceinline__ void sk_decode_stage(const unsigned char* tstage, uin
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
                 uint32_t s[8];
-                dq::lane_states<BITS, (CB != 2) ? 8 : 2>(reinterpret_cast<const uint32_t*>(tstage + krow * TROW_BYTES) + (2 * quarter + t) * NW, lane, s);
+                dq::lane_states<BITS, dq::tc_window_heavy<BITS, CB>()>(reinterpret_cast<const uint32_t*>(tstage + krow * TROW_BYTES) + (2 * quarter + t) * NW, lane, s);
                 dq::decode_frag<CB>(s, w[krow][t]);
             }
     }

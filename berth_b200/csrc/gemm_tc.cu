@@ -38,6 +38,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 
 namespace berth {
 namespace {
@@ -1421,13 +1422,19 @@ void had_r_128(const void* input, void* output, const void* scale, int pre_scale
 
 // CTAs of the dense kernel that run at once in clusters of `size` (0: such a cluster does not fit).  A cluster lies inside one
 // GPC, and how many SMs a GPC has differs: a B200 of 148 SMs does not hold 16 clusters of eight (their extra wave made a 421-row
-// 5120 x 1024 projection 30 us, clusters of four 20 us), so the driver is asked, once per device and size.
+// 5120 x 1024 projection 30 us, clusters of four 20 us).  For 148 SMs the numbers are cudaOccupancyMaxActiveClusters', written
+// down (three boards gave the same), because the split of K decides the order in which an output's partial sums are added: the
+// same shape has the same bits on every such GPU, whatever its GPCs look like (a board that holds fewer takes another wave).
+// Other SM counts ask the driver, once per device and size.
 static int cluster_slots(int size)
 {
     const int dev = current_device();
-    if (size == 1) return device_info(dev).sms;
-    static int known[kMaxDevices][9] = {};   // slots + 1
-    if (!known[dev][size]) {
+    const int sms = device_info(dev).sms;
+    if (size == 1) return sms;
+    static constexpr int k148[9] = {0, 148, 148, 135, 132, 130, 132, 105, 120};
+    if (sms == 148) return k148[size];
+    static std::atomic<int> known[kMaxDevices][9];   // slots + 1; threads that meet here store the same number
+    if (!known[dev][size].load()) {
         auto kern = k_exl3_gemm_tc<4, 2>;    // (every instance takes a whole SM)
         cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TGeo<4>::SMEM)), "gemm smem attribute");
         cudaLaunchConfig_t cfg = {};
@@ -1441,9 +1448,9 @@ static int cluster_slots(int size)
         cfg.numAttrs = 1;
         int n = 0;
         cuda_ok(cudaOccupancyMaxActiveClusters(&n, kern, &cfg), "cluster occupancy");
-        known[dev][size] = n * size + 1;
+        known[dev][size].store(n * size + 1);
     }
-    return known[dev][size] - 1;
+    return known[dev][size].load() - 1;
 }
 
 // Prefill linear for any row count > 32: rotate the activations, then the tensor-core GEMM.

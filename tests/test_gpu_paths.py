@@ -120,17 +120,21 @@ def test_router_tiles_bit_exact(oracle, T, H, E):
     assert (idx.cpu().numpy() == exp_idx).all()
     assert np.abs(tw.cpu().numpy() - exp_w).max() <= 1e-6
 
-@pytest.mark.parametrize("m,K,N,bits,cb,out_fp32", [(33, 512, 128, 4, 2, True), (64, 5120, 1024, 3, 2, False), (97, 2176, 384, 5, 0, True),
-                                                    (129, 4096, 256, 4, 1, False), (200, 1664, 640, 6, 2, False),
-                                                    (256, 2048, 128, 8, 2, True), (300, 5120, 256, 1, 2, False), (384, 3968, 128, 4, 2, True),
-                                                    (421, 5120, 1024, 4, 2, False), (40, 128, 128, 4, 2, True), (40, 384, 128, 4, 2, True)])
-def test_prefill_split_k(oracle, m, K, N, bits, cb, out_fp32):
-    """Few bands: the tile's K is split over a cluster (up to eight CTAs, uneven shares, passes without an owner's partner);
-    K below four stages per CTA is not."""
+@pytest.mark.parametrize("m,K,N,bits,cb,out_fp32,rows,split", [
+    (33, 512, 128, 4, 2, True, 128, 1), (64, 5120, 1024, 3, 2, False, 128, 8), (97, 2176, 384, 5, 0, True, 128, 8), (129, 4096, 256, 4, 1, False, 128, 8),
+    (200, 1664, 640, 6, 2, False, 128, 6), (256, 2048, 128, 8, 2, True, 128, 8), (300, 5120, 256, 1, 2, False, 128, 8), (384, 3968, 128, 4, 2, True, 128, 8),
+    (421, 5120, 1024, 4, 2, False, 128, 4), (40, 128, 128, 4, 2, True, 128, 1), (40, 384, 128, 4, 2, True, 128, 1),
+    (150, 2048, 1024, 4, 2, True, 256, 8), (300, 1024, 2176, 5, 2, False, 256, 3), (150, 1024, 2176, 3, 0, True, 256, 4), (300, 512, 6400, 4, 2, False, 384, 2)])
+def test_prefill_split_k(oracle, m, K, N, bits, cb, out_fp32, rows, split):
+    """Few bands: the tile's K is split over a cluster (up to eight CTAs, uneven shares, passes without an owner's partner, all
+    three tile heights); K below four stages per CTA is not.  On a GPU of 148 SMs the split follows from the shape."""
     w = synth.linear_weights(1234, f"split{K}{bits}", K, N, bits)
     x = synth.activations(1234, f"split{K}.x", m, K)
     c, _ = run_linear(x, w, bits, cb, out_fp32, prefill=True)
-    assert "k_exl3_gemm_tc" in kernels.prefill_lin.last_launch()
+    launch = kernels.prefill_lin.last_launch()
+    assert "k_exl3_gemm_tc" in launch
+    if kernels.device_sms(torch.cuda.current_device()) == 148:
+        assert f"grid={N // 128}x{-(-m // rows)}" + (f"x{split} " if split > 1 else " ") in launch and f"tile={rows}x" in launch
     assert_close(c, oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, cb), "split K")
     for _ in range(2):      # fixed order of the partial sums
         again, _ = run_linear(x, w, bits, cb, out_fp32, prefill=True)

@@ -27,8 +27,8 @@
 //               owns output column n = its TMEM lane; 128-point Hadamard over n by warp shuffles (strides
 //               1..16) and a shared-memory exchange between the four warps of the team (32, 64), output
 //               scale, coalesced stores.
-// Grouped launches (the experts of an MoE layer) take blockIdx.y as an index into a device-side
-// problem table {matrix of the stack, first row, rows}; the MMA then covers only the problem's rows
+// Grouped launches (the experts of an MoE layer) are a kernel of their own, k_exl3_gemm_tc_grouped: its items come from a
+// device-side problem table {matrix of the stack, first row, rows}, and the MMA covers only the problem's rows
 // (rounded up to 16), which is what makes small per-expert batches cheap.
 // All waits are bounded: a wait that runs out sets a status bit and the kernel carries on and
 // exits (wrong output, no hang).
@@ -394,14 +394,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int band = blockIdx.x;
-    int z = 0, m0 = blockIdx.y * (p.nsub_max * SUB), rows_here = min(p.m - m0, p.nsub_max * SUB);
-    if (p.problems) {
-        // (the table was written by kernels that completed before this launch)
-        if (int(blockIdx.y) >= min(max(__ldg(p.n_problems), 0), p.max_problems)) return;
-        const GemvProblem pr = load_problem(p.problems, blockIdx.y, p.n_matrices, p.nsub_max * SUB, p.m);
-        z = pr.z; m0 = pr.row0; rows_here = pr.rows;
-        if (rows_here < 1) return;
-    }
+    const int m0 = blockIdx.y * (p.nsub_max * SUB), rows_here = min(p.m - m0, p.nsub_max * SUB);
     const int row_end = m0 + rows_here;
     const int nsub = (rows_here + SUB - 1) / SUB;
     const int rows_pad = (rows_here + 15) & ~15;          // MMA N granularity
@@ -447,7 +440,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
             int sa = 0, pa = 0, st = 0, pt = 0;
             auto load_trellis = [&](int ks) {   // 4 k-tile rows of this band
                 mbar_arrive_expect_tx(full_t + 8 * st, T_STAGE_BYTES);
-                tma_load_3d(smem_u32(t_ring + st * T_STAGE_BYTES), &tmap_t, band * (TROW_BYTES / 8), (k0 + ks) * 4, z, full_t + 8 * st);
+                tma_load_3d(smem_u32(t_ring + st * T_STAGE_BYTES), &tmap_t, band * (TROW_BYTES / 8), (k0 + ks) * 4, 0, full_t + 8 * st);
                 if (++st == ST) { st = 0; pt ^= 1; }
             };
             // The first lap of the ring is asked into L2 while the rotation still runs, and read after the wait: a kernel before
@@ -455,7 +448,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
             // 40 / 421 rows: 222.8 / 494.8 us, with that copy 221.2 / 492.9, without the hint 229.3 / 493.0.)
             const int pre = min(kstages, ST);
             if (!p.defer_weights)
-                for (int ks = 0; ks < pre; ++ks) tma_prefetch_3d(&tmap_t, band * (TROW_BYTES / 8), (k0 + ks) * 4, z);
+                for (int ks = 0; ks < pre; ++ks) tma_prefetch_3d(&tmap_t, band * (TROW_BYTES / 8), (k0 + ks) * 4, 0);
             pdl_wait();
             for (int ks = 0; ks < pre; ++ks) load_trellis(ks);
             for (int ks = 0; ks < kstages; ++ks) {
@@ -532,7 +525,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemm_tc(const __grid_const
         const int quarter = warp & 3;
         const int n = quarter * 32 + lane;
         pdl_wait();   // svh may be the output of a kernel that is still running (the rotation before this launch triggers at its start)
-        const float scale = __half2float(p.svh[size_t(z) * p.n + band * BN + n]);
+        const float scale = __half2float(p.svh[band * BN + n]);
         mbar_wait_parked(acc_full, 0, p.status, team == 0 ? 1000 : 100);
         tc_fence_after();
         // per team: transposition buffer and the band's scales, in the activation ring, which is idle by now

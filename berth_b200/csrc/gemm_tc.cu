@@ -1410,8 +1410,8 @@ __global__ void __launch_bounds__(256) k_rotate_rows_plain(const RotateArgs a)
 }
 }  // namespace
 
-void had_r_128(const void* input, void* output, const void* scale, int pre_scale, int rows, int cols, int fp32,
-               cudaStream_t stream);
+const char* had_r_128(const void* input, void* output, const void* scale, int pre_scale, int rows, int cols, int fp32,
+                      cudaStream_t stream);
 
 // CTAs of the dense kernel that run at once in clusters of `size` (0: such a cluster does not fit).  A cluster lies inside one
 // GPC, and how many SMs a GPC has differs: a B200 of 148 SMs does not hold 16 clusters of eight (their extra wave made a 421-row
@@ -1453,7 +1453,7 @@ std::string launch_gemm_tc(const void* a, const void* trellis, void* c, const vo
 {
     if (size_k % 128 != 0)
         throw std::runtime_error("exl3 linear: no linked kernel for size_k that is not a multiple of 128 (128-wide Hadamard)");
-    had_r_128(a, a_had, suh, 1, size_m, size_k, 0, stream);
+    const std::string rotation = had_r_128(a, a_had, suh, 1, size_m, size_k, 0, stream);
     GemmArgs args;
     args.c = c;
     args.svh = static_cast<const __half*>(svh);
@@ -1493,7 +1493,7 @@ std::string launch_gemm_tc(const void* a, const void* trellis, void* c, const vo
             }
     }
     launch_tc_bits(k_bits, codebook, a_had, trellis, args, stream);
-    return "k_had128<f16,pre> + k_exl3_gemm_tc<" + std::to_string(k_bits) + "," + std::to_string(codebook) + "> grid=" +
+    return rotation + " + k_exl3_gemm_tc<" + std::to_string(k_bits) + "," + std::to_string(codebook) + "> grid=" +
            std::to_string(size_n / BN) + "x" + std::to_string((size_m + args.nsub_max * SUB - 1) / (args.nsub_max * SUB)) +
            (args.split > 1 ? "x" + std::to_string(args.split) : "") + " block=" + std::to_string(kThreads) + " tile=" + std::to_string(args.nsub_max * SUB) + "x128x64 tmem=512";
 }
@@ -1511,7 +1511,7 @@ std::string launch_gemm_tc_splitk(const void* a, const void* trellis, void* c, c
     const size_t per_cta = size_t(2) * kSkRows * BN * sizeof(float);
     if (size_t(grid) * per_cta > sc.slab_bytes) grid = int(sc.slab_bytes / per_cta);
     if (grid < 1) throw std::runtime_error("exl3 linear: split-K scratch is too small for this shape");
-    had_r_128(a, a_had, suh, 1, size_m, size_k, 0, stream);
+    const std::string rotation = had_r_128(a, a_had, suh, 1, size_m, size_k, 0, stream);
     SplitKArgs args;
     args.defer_weights = weights_streamed() ? 1 : 0;
     args.c = c;
@@ -1526,7 +1526,7 @@ std::string launch_gemm_tc_splitk(const void* a, const void* trellis, void* c, c
     const bool shared = units % grid != 0 || (units / grid) % (size_k / BK) != 0;
     if (shared)
         launch_pdl(k_sk_finish, dim3(size_n / BN, (size_m + 3) / 4), dim3(128), 0, stream, "k_sk_finish launch", args);
-    return "k_had128<f16,pre> + k_exl3_gemm_tc_splitk<" + std::to_string(k_bits) + "," + std::to_string(codebook) + "> grid=" +
+    return rotation + " + k_exl3_gemm_tc_splitk<" + std::to_string(k_bits) + "," + std::to_string(codebook) + "> grid=" +
            std::to_string(grid) + " block=" + std::to_string(kThreads) + " stage=64x128 rows=" + std::to_string((size_m + 15) / 16 * 16) +
            (shared ? " + k_sk_finish" : "");
 }

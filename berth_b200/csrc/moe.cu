@@ -902,8 +902,9 @@ void check_moe_shapes(const berth_moe_weights* w, int T, bool routes = false)
     if (w->codebook < 0 || w->codebook > 2) throw std::runtime_error("moe: codebook must be 0, 1, or 2");
 }
 
-void router_topk(const void* x, const void* w_router, const float* bias, int32_t* topk_idx, float* topk_w, float* logits,
-                 int T, int H, int E, int k, cudaStream_t st)
+// Returns the names of the kernels that run.
+std::string router_topk(const void* x, const void* w_router, const float* bias, int32_t* topk_idx, float* topk_w, float* logits,
+                        int T, int H, int E, int k, cudaStream_t st)
 {
     const size_t smem = size_t(kRouterTok) * H * 4 + size_t(32) * kRouterTok * 33 * 4;
     if (smem > 200 * 1024) throw std::runtime_error("moe router: hidden is too large for the router's shared-memory tile");
@@ -916,7 +917,10 @@ void router_topk(const void* x, const void* w_router, const float* bias, int32_t
     }
     const dim3 rgrid(E / 32, (T + kRouterTok - 1) / kRouterTok);
     const size_t smem_wide = size_t(kRouterTok) * H * 4 + size_t(16) * kRouterTok * kWidePitch * 4;
+    std::string name;
     auto narrow = [&](auto kern, int warps, int tok) {
+        name = "k_moe_router_logits<" + std::to_string(warps) + "," + std::to_string(tok) + "> grid=" + std::to_string(E / 32) + "x" +
+               std::to_string((T + tok - 1) / tok);
         const size_t bytes = size_t(tok) * H * 4 + size_t(32) * tok * 33 * 4;
         launch_pdl(kern, dim3(E / 32, (T + tok - 1) / tok), dim3(warps * 32), bytes, st, "k_moe_router_logits launch", (const __half*) x,
                    (const __half*) w_router, bias, logits, T, H, E);
@@ -930,6 +934,7 @@ void router_topk(const void* x, const void* w_router, const float* bias, int32_t
         }
         launch_pdl(k_moe_router_logits_wide, dim3(E / 128, rgrid.y), dim3(512), smem_wide, st, "k_moe_router_logits_wide launch",
                    (const __half*) x, (const __half*) w_router, bias, logits, T, H, E);
+        name = "k_moe_router_logits_wide grid=" + std::to_string(E / 128) + "x" + std::to_string(rgrid.y);
     } else if (one_wave(1)) narrow(k_moe_router_logits<32, 1>, 32, 1);
     else if (one_wave(2)) narrow(k_moe_router_logits<32, 2>, 32, 2);
     else if (one_wave(4)) narrow(k_moe_router_logits<32, 4>, 32, 4);
@@ -938,6 +943,7 @@ void router_topk(const void* x, const void* w_router, const float* bias, int32_t
     cuda_ok(cudaGetLastError(), "k_moe_router_logits launch");
     launch_pdl(E <= 128 ? k_moe_topk<4> : (E <= 256 ? k_moe_topk<8> : k_moe_topk<32>), dim3((T + 3) / 4), dim3(128), 0, st, "k_moe_topk launch", logits, topk_idx, topk_w, T, E, k);
     cuda_ok(cudaGetLastError(), "k_moe_topk launch");
+    return name + " + k_moe_topk";
 }
 
 // keys[n] -> counts/offsets/problems + perm/inv; experts [e0, e0 + n_local).
@@ -1107,8 +1113,7 @@ extern "C" int berth_moe_router_topk(const void* x, const void* w_router, const 
         if (n_experts < 32 || n_experts % 32 || n_experts > 1024)
             throw std::runtime_error("moe router: n_experts must be a multiple of 32 up to 1024");
         if (top_k < 1 || top_k > 32 || top_k > n_experts) throw std::runtime_error("moe router: top_k must be in 1..=32");
-        router_topk(x, w_router, router_bias, topk_idx, topk_w, logits, T, hidden, n_experts, top_k, (cudaStream_t) stream);
-        st.launch = "k_moe_router_logits grid=" + std::to_string(n_experts / 32) + "x" + std::to_string((T + kRouterTok - 1) / kRouterTok) + " + k_moe_topk";
+        st.launch = router_topk(x, w_router, router_bias, topk_idx, topk_w, logits, T, hidden, n_experts, top_k, (cudaStream_t) stream);
     });
 }
 
@@ -1315,7 +1320,7 @@ extern "C" int berth_moe_ep_experts(const berth_moe_weights* w, const void* recv
             cuda_ok(cudaGetLastError(), "k_moe_gather launch");
         }
         if (TS) cuda_ok(cudaMemcpyAsync(ysh, yr + size_t(n_rows) * H, size_t(TS) * H * 2, cudaMemcpyDeviceToDevice, cs), "moe ep experts: shared output copy");
-        st.launch = "k_moe_segment_scan/keys + k_moe_count/scan/scatter + k_moe_gather_rows + 3 x (" + st.launch + ") + k_silu_mul + k_moe_gather_n";
+        st.launch = "k_moe_segment_scan/keys + k_moe_count/scan/scatter + k_moe_gather_rows + " + st.launch + " + k_moe_gather_n";
     });
 }
 
@@ -1480,7 +1485,7 @@ extern "C" int berth_moe_p2p_experts(const berth_moe_weights* w, const void* x_l
             k_rows_from_offset<<<std::min(TS, 148 * 8), 256, 0, cs>>>(yr, (__half*) ysh, es.offsets + NL, TS, H, max_rows);
             cuda_ok(cudaGetLastError(), "k_rows_from_offset launch");
         }
-        st.launch = "k_moe_scan + 3 x (" + st.launch + ") + k_silu_mul_rows + k_ep_return + k_ep_barrier";
+        st.launch = "k_moe_scan + " + st.launch + " + k_ep_return + k_ep_barrier";
     });
 }
 
@@ -1538,7 +1543,7 @@ extern "C" int berth_moe_layer(const berth_moe_weights* w, const void* x, int T,
         ExpertScratch es = carve_experts(b, RT, NM, H, I, plan);
         b += carve_experts(nullptr, R + T, E + 1, H, I, plan).bytes;
 
-        router_topk(x, w->w_router, w->router_bias, topk_idx, topk_w, logits, T, H, E, K, cs);
+        const std::string router = router_topk(x, w->w_router, w->router_bias, topk_idx, topk_w, logits, T, H, E, K, cs);
         const bool paired = up_behind_gate(w, NM);
         dispatch(topk_idx, R, 0, E, plan.chunk, es, perm, inv, cs, fused_shared ? T : 0, paired ? RT : 0, NM);
         // the rotation kernel of gate and up gathers the routed rows (and the shared expert's) from x itself
@@ -1567,7 +1572,7 @@ extern "C" int berth_moe_layer(const berth_moe_weights* w, const void* x, int T,
         }
         launch_pdl(k_moe_combine, dim3(T, (H + 511) / 512), dim3(256), 0, cs, "k_moe_combine launch", yr, inv, topk_w, ysh, (float*) out, H, K, R);
         cuda_ok(cudaGetLastError(), "k_moe_combine launch");
-        st.launch = std::string("k_moe_router_logits + k_moe_topk + ") + (R <= kSmallKeys ? "k_moe_dispatch_small" : "k_moe_count/scan/scatter") +
+        st.launch = router + " + " + (R <= kSmallKeys ? "k_moe_dispatch_small" : "k_moe_count/scan/scatter") +
                     " + " + st.launch + " + k_moe_combine" + (fused_shared ? " [shared expert as matrix E of the grouped launches]" : "");
     });
 }

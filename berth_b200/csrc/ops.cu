@@ -383,8 +383,9 @@ void reconstruct(void* unpacked, const void* packed, int size_k, int slice_n, in
     cuda_ok(cudaPeekAtLastError(), "k_trellis_decode");
 }
 
-void had_r_128(const void* input, void* output, const void* scale, int pre_scale, int rows, int cols, int fp32,
-               cudaStream_t stream)
+// Returns the name of the kernel that runs.
+const char* had_r_128(const void* input, void* output, const void* scale, int pre_scale, int rows, int cols, int fp32,
+                      cudaStream_t stream)
 {
     if (cols % 128 != 0) throw std::runtime_error("prefill had_r_128: had columns must be a multiple of 128");
     if (rows < 1) throw std::runtime_error("prefill had_r_128: rows must be positive");
@@ -398,6 +399,7 @@ void had_r_128(const void* input, void* output, const void* scale, int pre_scale
     if (!fp32 && pre_scale && scale && aligned && total >= 148LL * 64) {
         const int wide = int(std::min<long long>((total + 15) / 16, 148LL * 16));
         launch_pdl(k_had128_wide, dim3(wide), dim3(128), 0, stream, "k_had128", static_cast<const __half*>(input), static_cast<__half*>(output), sc, total, bpr);
+        return "k_had128_wide";
     } else if (fp32) {
         if (pre_scale) launch_pdl(k_had128<true, true>, dim3(grid), dim3(128), 0, stream, "k_had128", input, output, sc, rows, bpr);
         else launch_pdl(k_had128<true, false>, dim3(grid), dim3(128), 0, stream, "k_had128", input, output, sc, rows, bpr);
@@ -405,6 +407,7 @@ void had_r_128(const void* input, void* output, const void* scale, int pre_scale
         if (pre_scale) launch_pdl(k_had128<false, true>, dim3(grid), dim3(128), 0, stream, "k_had128", input, output, sc, rows, bpr);
         else launch_pdl(k_had128<false, false>, dim3(grid), dim3(128), 0, stream, "k_had128", input, output, sc, rows, bpr);
     }
+    return fp32 ? (pre_scale ? "k_had128<f32,pre>" : "k_had128<f32,post>") : (pre_scale ? "k_had128<f16,pre>" : "k_had128<f16,post>");
 }
 
 }  // namespace berth
@@ -431,8 +434,7 @@ extern "C" int berth_prefill_had_r_128(const void* input, void* output, const vo
     CallState& st = prefill_state();
     return guarded(st, [&] {
         if (!input || !output) throw std::runtime_error("prefill had_r_128: null device pointer");
-        had_r_128(input, output, scale, pre_scale, rows, cols, fp32, (cudaStream_t) stream);
-        st.launch = std::string("k_had128<") + (fp32 ? "f32" : "f16") + (pre_scale ? ",pre" : ",post") + "> block=128";
+        st.launch = std::string(had_r_128(input, output, scale, pre_scale, rows, cols, fp32, (cudaStream_t) stream)) + " block=128";
     });
 }
 

@@ -7,6 +7,7 @@ pytestmark = pytest.mark.gpu
 
 from berth_b200 import Codebook, OutDtype, kernels, moe, synth   # noqa: E402
 from tests.gpu_util import assert_close, dev, run_linear   # noqa: E402
+from tests.test_gpu_parity import test_rms_norm_bit_exact as rms_norm_bit_exact   # noqa: E402
 
 
 def test_integer_path_one_hot_blocks(oracle):
@@ -99,6 +100,7 @@ def test_moe_layer_few_tokens_vs_oracle(oracle, T, bits, inter, shared, E):
         layer.forward(dev(x), out, idx, w)
         torch.cuda.synchronize()
         assert kernels.device_status(torch.cuda.current_device()) == 0
+        assert ("fused,grouped" in moe.last_launch()) == (T <= 4)
         _, exp_idx, exp_w = oracle.moe_layer(wts, x)
         assert (idx.cpu().numpy() == exp_idx).all()
         assert_close(out.cpu().numpy(), oracle.moe_layer_f64(wts, x, exp_idx, exp_w), f"T={T} pair={pair}")
@@ -114,6 +116,8 @@ def test_router_tiles_bit_exact(oracle, T, H, E):
     logits = torch.empty((T, E), dtype=torch.float32, device="cuda")
     moe.router_topk(dev(x), dev(w), None, idx, tw, logits, T, H, E, k)
     torch.cuda.synchronize()
+    tok = next((t for t in (1, 2, 4, 8) if E // 32 * -(-T // t) <= kernels.device_sms(torch.cuda.current_device())), 8)
+    assert f",{tok}> grid={E // 32}x{-(-T // tok)} " in moe.last_launch()
     exp_logits = oracle.router_logits(x, w)
     exp_idx, exp_w = oracle.router_topk(exp_logits, k)
     assert (logits.cpu().numpy().view(np.uint32) == exp_logits.view(np.uint32)).all()
@@ -152,6 +156,7 @@ def test_rotation_of_many_rows_bit_exact(oracle, rows, K, skip):
     out = torch.empty((rows, K), dtype=torch.float16, device="cuda")
     kernels.prefill_lin.had_r_128(buf[skip:], out, dev(w["suh"]), True, rows, K, False)
     torch.cuda.synchronize()
+    assert ("k_had128_wide" in kernels.prefill_lin.last_launch()) == (skip == 0)
     assert (out.cpu().numpy().view(np.uint16) == oracle.had_r_128(x, w["suh"], True).view(np.uint16)).all()
 
 
@@ -165,6 +170,7 @@ def test_silu_mul_every_gate_value_bit_exact(oracle, n, limit, skip):
     out = torch.empty(n, dtype=torch.float16, device="cuda")
     kernels.ops.silu_mul(g[skip:], u[skip:], out, n, limit)
     torch.cuda.synchronize()
+    assert ("k_silu_mul_wide" in kernels.ops.last_launch()) == (n == 65536 * 16 and skip == 0)
     got, exp = out.cpu().numpy(), oracle.silu_mul(gate, up, limit)
     nan = np.isnan(exp)
     assert (np.isnan(got) == nan).all()
@@ -303,3 +309,10 @@ def test_moe_layer_8_bits_tensor_core_stage(oracle, H, inter):
     _, exp_idx, exp_w = oracle.moe_layer(wts, x)
     assert (idx.cpu().numpy() == exp_idx).all()
     assert_close(out.cpu().numpy(), oracle.moe_layer_f64(wts, x, exp_idx, exp_w), "8 bits")
+
+
+@pytest.mark.parametrize("rows,dim", [(2, 2048), (2, 2052), (1, 3000), (3, 4096), (1, 4100), (2, 6148), (3, 8192), (2, 8196), (1, 12288)])
+@pytest.mark.parametrize("wbf", [True, False])
+def test_rms_norm_groups_in_registers(oracle, rows, dim, wbf):
+    """4, 8, 12 or 16 groups of four per thread held in registers, at the edges of each, and the loop above 8192 columns."""
+    rms_norm_bit_exact(oracle, rows, dim, wbf)

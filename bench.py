@@ -173,12 +173,13 @@ class DecodeStack:
         # one row: gate+up (one stacked integer-path launch, rotation and finishing inside it), down (the same kernel, with
         # silu(gate) * up formed in its rotation) and o (one launch each), q/k/v (the same kernel over the three matrices,
         # one launch) = 4 launches.
-        # two rows: down and o as k_exl3_gemv (rotation inside) + k_gemv_finish = 6; three: k_rotate_in in front of them = 8.
-        # four rows: the same, with k_rotate_in_i8 per stacked matrix before the stacked launch (its limb tiles do not fit) = 10.
+        # two rows: o as k_exl3_gemv (rotation inside) + k_gemv_finish = 5; three rows as one.
+        # four rows: down and o as k_rotate_in + k_exl3_gemv + k_gemv_finish, and k_rotate_in_i8 per stacked matrix before the stacked
+        # launch (its limb tiles do not fit) = 10.
         # 5..16 rows: gate, up, down, o with three launches each (k_rotate_in + k_exl3_gemv + k_gemv_finish), q/k/v as one
         # sliced launch of the fp16-path kernel (k_rotate_in + k_exl3_gemv + k_gemv_finish) = 15.
         # above: the same with k_had128 + k_exl3_gemm_tc_splitk + k_sk_finish per linear, and k_silu_mul = 16.
-        self.launches_per_step = {1: 4, 2: 6, 3: 8, 4: 10}.get(m, 15 if m <= 16 else 16)
+        self.launches_per_step = {1: 4, 2: 5, 3: 4, 4: 10}.get(m, 15 if m <= 16 else 16)
 
     def step(self, i: int) -> None:
         from berth_b200.kernels import OutDtype

@@ -253,8 +253,8 @@ bool gemv_i8_grouped_fits(long long most, int rows, int size_k, int size_n, int 
 std::string launch_gemv_i8_grouped(const GroupedI8& g, int rows, int size_k, int size_n, int k_bits, const GemvScratch& sc, int sms,
                                    cudaStream_t stream);
 
-// True when launch_gemv hands this dense MUL1 linear to launch_gemv_i8.
-bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc);
+// True when launch_gemv hands this dense MUL1 linear (`silu`: with silu(gate) * up formed in its rotation) to launch_gemv_i8.
+bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc, bool silu);
 
 constexpr float kRScale = 0.088388347648f;  // 1/sqrt(128), csrc/prefill_lin/reconstruct.cu:43-44
 

@@ -669,7 +669,7 @@ std::string launch_gemv(const void* a, const void* trellis, void* c, const void*
     if (k_bits < 1 || k_bits > 8) throw std::runtime_error("exl3 linear: K must be in 1..=8");
     // MUL1, one row, and two to four where it pays: integer tensor path with the weights in tensor memory.  The 6 bpw lm_head
     // (5120 x 248320: every CTA holds thirteen whole band groups) takes 334 us there and 414 us here; a 5120 x 6144 linear of 4 bpw 14.1 us.
-    if (codebook == 2 && gemv_i8_serves(size_m, size_k, size_n, k_bits, sms, sc))
+    if (codebook == 2 && gemv_i8_serves(size_m, size_k, size_n, k_bits, sms, sc, act.up != nullptr))
         return launch_gemv_i8(a, trellis, c, suh, a_had, svh, size_m, size_k, size_n, k_bits, out_fp32, sc, sms, stream, argmax, 1, residual, sample, act);
     const int tg = size_m <= 8 ? 1 : (size_m <= 16 ? 2 : 4);
     const int bu = k_bits <= 4 ? 2 : 1;   // bands per unit, as Geo<BITS, TG>::BU

@@ -218,7 +218,8 @@ __device__ __forceinline__ float quantise_block(const float (&hv)[4], int lane, 
 }
 
 // ---------------------------------------------------------------- the kernel
-// FUSED (one group of four rows, dense launches in which the limb tiles of every CTA's units fit the limb area): no rotation kernel runs before this one and no limb tile travels through L2; while the first weight
+// FUSED (one group of four rows; the limb tiles of every CTA's units fit the limb area, and for a stack the rotation is short enough):
+// no rotation kernel runs before this one and no limb tile travels through L2; while the first weight
 // stages are in flight the decoding and epilogue warps rotate and quantise the 128-block of every unit of the CTA
 // into a shared-memory area of its own (tiles of 2 * rows limb rows, a quarter of the ring-stage tile for one row),
 // and the CTAs that hold band group 0 also write the rotated activations and block sums for the caller and the
@@ -699,7 +700,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_exl3_gemv_i8(const __grid_const
 
 // ---------------------------------------------------------------- rotation + quantisation of the activations
 // One warp per (row, 128-block): a_had = fp16(H128(a * suh) / sqrt(128)) into the caller's buffer (bit-exact
-// with the other paths); then the block's fixed-point form: scale = max|a_had| / 32512, v = rint(a_had / scale),
+// with the other paths); then the block's fixed-point form, of the values before that rounding: scale = max|a| / 32512, v = rint(a / scale),
 // v = 256 hi + lo with hi in [-127, 127], lo in [-128, 127].  Each limb is written replicated over the four
 // bytes of a 32-bit word (the four u8 k-slots of a weight's product) at its place in the limb tile of the
 // block: [MMA k-step 16][row group nb][core matrix 2][limb row 8][16 bytes], limb row = 2 * (row % 4) + (0 high,
@@ -818,33 +819,39 @@ static bool stack_rotates_in_kernel(int k_bits, int rows, long long tiles)
     return tiles <= fused_max_units(k_bits, rows) && (rows % 2 != 0 || rows * tiles <= 80);
 }
 
-// Two to four rows of one matrix: whether this kernel is at least as fast as k_exl3_gemv with its rotation (from three rows on a
-// launch of its own) and finishing launches.  Both were timed for 111 matrices from 128 x 512 to 17408 x 17408 at 2, 3, 4, 5, 6
-// and 8 bits, weights out of cache.  This kernel rotates rows * (128-blocks of a CTA) blocks before its first MMA and saves launches; its
-// decode is ahead where a unit is one band (5 bits and more) and level below.  So, with `units` = units of a CTA:
-//  - up to 4 bits: where a CTA holds whole band groups and meets few 128-blocks (128 x 6144, two rows: 4.0 against 5.4 us), where K
-//    is so short that the launches are everything (kblocks <= 4), and at 4 bits for a vocabulary's width (5120 x 151552,
-//    two rows: 160 against 166 us).  Elsewhere it loses: 5120 x 1024, four rows: 14.2 against 11.3 us;
-//  - from 5 bits on: whole band groups (5120 x 151552 at 6 bits, three rows: 209 against 254 us; with four rows from one and a half or two of them a CTA),
-//    few bands (5120 x 1024, four rows: 9.3 against 11.6), three rows of all but short matrices (5120 x 6144: 17.1 against 20.0),
-//    four while the rotation is short; two rows only where the other kernel cannot rotate in the launch itself (more than 26
-//    units; 5120 x 6144: 17.6 against 15.5).
-// No point of the sweep is more than 2.5 % slower here than there, and five of 920 are more than 1 %.
-static bool few_rows_pay(int rows, int k_bits, long long units, int kblocks, bool few_bands)
+// Two to four rows of one matrix: whether to take this kernel instead of k_exl3_gemv, which from three rows on needs a rotation
+// launch and always a finishing launch.  Timed in a stream, weights out of cache: 111 matrices from 128 x 512 to 17408 x 17408 at 2
+// to 8 bits, the same linear back to back (there the other kernel's launches overlap with their neighbours), and as o and down of
+// transformer layers of 1024 to 5120 (there each of its launches costs 1-2 us: o of three rows, 6144 x 5120 at 4 bits behind its
+// q/k/v, 43.1 against 41.0 us).  This kernel rotates rows * (128-blocks of a CTA) blocks before its first MMA; its decode is ahead where
+// a unit is one band (5 bits and more) and level below.  It is taken where the layers gain and the linear by itself is not
+// slower than the fp16 path by more than a few percent; `units` = units of a CTA:
+//  - down with silu in its rotation (it follows gate and up directly): two and three rows (a long one of fewer than 4 bits not), four
+//    while the rotation is short;
+//  - up to 4 bits: where K is so short that the launches are everything, three rows of matrices with enough bands (8192 x 6144: 18.8
+//    against 19.5 us), two of few bands, and a vocabulary's width at 4 bits (5120 x 151552, two rows: 160 against 166 us).  Few bands
+//    and three or four rows lose (2048 x 1024 at 4 bits, four rows: 13.7 against 11.9 us; 17408 x 6144, four rows: 37.1 against 32.7);
+//  - from 5 bits on: whole band groups (5120 x 151552 at 6 bits, three rows: 209 against 254 us), few bands (5120 x 1024, four rows:
+//    8.9 against 11.6), three rows of all but short matrices (5120 x 6144: 16.0 against 20.0), four while the rotation is short; two
+//    rows only while it is a single block or two, or where the other kernel cannot rotate in the launch itself (more than 26 units).
+static bool few_rows_pay(int rows, int k_bits, long long units, int kblocks, bool few_bands, bool silu)
 {
     const bool whole = units >= kblocks;
-    if (k_bits <= 4)
-        return (whole && (kblocks <= (rows == 2 ? 16 : 2) || (k_bits == 4 && rows < 4 && units >= 4LL * kblocks))) ||
-               (kblocks <= 4 && (few_bands || units >= 4LL * kblocks));
-    if (whole) return rows < 4 || kblocks <= 2 || units >= 2LL * kblocks || (kblocks <= 16 && 2 * units >= 3LL * kblocks);
-    if (few_bands) return true;
-    if (rows == 2) return units > 26 && units <= 50;
-    return rows == 3 ? kblocks >= 8 : (kblocks >= 16 || 2 * units < kblocks) && units < 10;
+    if (silu && (rows == 2 || units < 10)) return true;
+    if (silu && rows == 3 && k_bits <= 4) return k_bits == 4 || units < 16;
+    if (k_bits <= 4) {
+        if (whole) return kblocks <= (rows == 2 ? 16 : 2) || (k_bits == 4 && rows < 4 && units >= 4LL * kblocks) || (kblocks <= 4 && units >= 4LL * kblocks);
+        if (few_bands) return rows == 2 || kblocks <= 8;
+        return rows == 3 && kblocks >= 8 && units >= 3 && 2 * units <= kblocks;
+    }
+    if (whole || few_bands) return true;
+    if (rows == 2) return (units <= 3 && kblocks >= 8) || units > 26;
+    return kblocks >= 8 && (rows == 3 || units < 15);
 }
 
 // Whether launch_gemv sends a dense MUL1 linear here: it pays, the rotation fits the kernel and the scratch suffices (where it
 // does not, the fp16-path kernel still serves the shape).
-bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc)
+bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, const GemvScratch& sc, bool silu)
 {
     if (size_m < 1 || size_m > 4 || size_k % 128 != 0 || size_n % 128 != 0 || k_bits < 1 || k_bits > 8) return false;
     const int bu = k_bits <= 4 ? 2 : 1;
@@ -854,7 +861,7 @@ bool gemv_i8_serves(int size_m, int size_k, int size_n, int k_bits, int sms, con
     if (grid < 1) return false;
     const long long units_per_cta = (units + grid - 1) / grid;
     if (std::min<long long>(units_per_cta, kblocks) > fused_max_units(k_bits, size_m)) return false;
-    if (size_m > 1 && !few_rows_pay(size_m, k_bits, units_per_cta, kblocks, grid < sms)) return false;
+    if (size_m > 1 && !few_rows_pay(size_m, k_bits, units_per_cta, kblocks, grid < sms, silu)) return false;
     return size_t(bgroups) <= sc.counter_words && size_t(size_m) * kblocks <= sc.blocksum_floats &&
            size_t(kblocks) * (size_t(16) * 256 + 128) <= sc.afrag_bytes &&
            size_t(grid) * 2 * (size_t(size_m) * bu * 128 + 32) * sizeof(float) <= sc.slab_bytes;

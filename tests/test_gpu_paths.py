@@ -58,9 +58,10 @@ def test_integer_path_several_band_groups_per_cta(oracle, K, N, bits):
     assert kernels.device_status(torch.cuda.current_device()) == 0
 
 @pytest.mark.parametrize("m,K,N,bits,here", [(m, K, N, bits, m in where) for K, N, bits, where in [
-    (5120, 1024, 4, ()), (5120, 1024, 5, (2, 3, 4)), (2176, 3072, 5, (3, 4)), (1024, 6144, 5, (3, 4)), (1024, 8192, 6, (3,)), (896, 8192, 6, ()), (128, 128 * 301, 6, (2, 3, 4)),
-    (384, 128 * 301, 5, (2, 3, 4)), (384, 128 * 200, 6, (2, 3, 4)), (2048, 128 * 200, 6, (2, 3)), (1152, 640, 3, ()), (384, 640, 3, (2, 3, 4)), (256, 128 * 301, 4, (2, 3, 4)),
-    (2048, 128 * 301, 4, (2,)), (2176, 128 * 301, 4, ()), (3584, 128 * 130, 5, (3,)), (1024, 128 * 240, 5, (2, 3, 4)), (2048, 128 * 100, 8, (3,))] for m in (2, 3, 4)])
+    (5120, 1024, 4, (2,)), (5120, 1024, 5, (2, 3, 4)), (2176, 3072, 5, (2, 3, 4)), (1024, 128 * 80, 6, (3, 4)), (896, 8192, 6, ()),
+    (128, 128 * 301, 6, (2, 3, 4)), (384, 128 * 301, 5, (2, 3, 4)), (2048, 128 * 100, 8, (3, 4)), (1152, 640, 3, (2,)), (1024, 640, 3, (2, 3, 4)),
+    (256, 128 * 301, 4, (2, 3, 4)), (2048, 128 * 301, 4, (2,)), (2176, 128 * 301, 4, ()), (3584, 128 * 130, 5, (3,)), (2048, 6144, 3, (3,)),
+    (2048, 128 * 96, 4, (3,)), (3072, 3072, 4, ()), (3072, 6400, 3, (3,))] for m in (2, 3, 4)])
 def test_integer_path_two_to_four_rows(oracle, m, K, N, bits, here):
     """Both sides of each line of the rule that picks the kernel."""
     w = synth.linear_weights(1234, f"few{K}{bits}", K, N, bits)
@@ -69,6 +70,18 @@ def test_integer_path_two_to_four_rows(oracle, m, K, N, bits, here):
     assert ("k_exl3_gemv_i8" in kernels.last_launch()) == here and ("fused" in kernels.last_launch() or not here)
     assert_close(c, oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, 2), "few rows")
     assert (ah == oracle.had_r_128(x, w["suh"], True).view(np.uint16)).all()
+
+@pytest.mark.parametrize("m,K,N,bits,here", [(2, 5120, 4096, 4, True), (3, 5120, 2048, 4, True), (3, 10240, 8192, 4, True), (3, 10240, 8192, 3, False), (4, 5120, 2048, 4, True), (4, 5120, 8192, 5, False)])
+def test_integer_path_two_to_four_rows_silu(oracle, m, K, N, bits, here):
+    """The down projection's rule: silu(gate) * up in the rotation, short and long ones."""
+    w = synth.linear_weights(1234, f"fewsilu{K}{N}", K, N, bits)
+    gate, up = (synth.activations(1234, f"fewsilu.{c}{m}", m, K) for c in "gu")
+    c, ah = torch.empty((m, N), dtype=torch.float32, device="cuda"), torch.empty((m, K), dtype=torch.float16, device="cuda")
+    kernels.exl3_linear_silu(dev(gate), dev(up), dev(w["trellis"]), c, dev(w["suh"]), ah, dev(w["svh"]), m, K, N, bits, Codebook(2), OutDtype.F32)
+    torch.cuda.synchronize()
+    assert ("k_exl3_gemv_i8" in kernels.last_launch()) == here
+    x = oracle.silu_mul(gate.ravel(), up.ravel(), 0.0).view(np.float16).reshape(m, K)
+    assert_close(c.cpu().numpy(), oracle.linear_f64(x, w["trellis"], w["suh"], w["svh"], K, N, bits, 2), "silu")
 
 @pytest.mark.parametrize("m,N,inside", [(2, 128 * 720, True), (2, 128 * 760, False), (3, 128 * 720, True), (4, 128 * 360, True), (4, 128 * 380, False)])
 def test_stack_rotation_inside_or_before(oracle, m, N, inside):

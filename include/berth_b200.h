@@ -33,7 +33,8 @@
  * streams) must not share it: berth drives one stream per device, and so must every other caller.
  * The prefill kernels use none of it.  The kernels of one linear are chained by programmatic
  * dependent launch: a decode kernel may prefetch weights while the kernel before it on the stream
- * still runs, so the trellis must not be written by the kernel that directly precedes a linear.
+ * still runs, so the trellis must not be written by the kernel that directly precedes a linear of up
+ * to 32 rows (the prefill kernels read it after their predecessor ended).
  */
 #ifndef BERTH_B200_H
 #define BERTH_B200_H
@@ -48,12 +49,14 @@ extern "C" {
 /* ------------------------------------------------------------------ decode linear (m >= 1)
  * Replaces berth_exl3_linear (crates/berth-kernels/src/ffi.rs:7-21,
  * crates/berth-kernels/csrc/linear.cu:209-286,362-394): c = H(H(a*suh) . W(trellis)) * svh.
- * Serves every size_m: one row of a MUL1 matrix on the integer-path decode kernel (codebook byte sums in tensor
- * memory, tcgen05.mma kind::i8, rotation and finishing inside the kernel); up to 16 rows (and up to 32 of a small
- * matrix) the fused decode GEMV; 17..32 rows of a large matrix the persistent split-K tensor-core kernel; above, the
- * tiled tcgen05 tensor-core GEMM.  berth_exl3_last_launch names the kernels that ran.  Programmatic-launch contract:
- * the kernels start fetching `trellis` while the kernel before them on the stream may still be running, so the
- * weights must be final before that kernel starts; every other tensor is touched only after the predecessor ended. */
+ * Serves every size_m: one row of a MUL1 matrix, and two to four where it is measured to pay, on the integer-path decode
+ * kernel (codebook byte sums in tensor memory, tcgen05.mma kind::i8, rotation and finishing inside the kernel); else up
+ * to 16 rows (and up to 32 of a small matrix) the fused decode GEMV; 17..32 rows of a large matrix the persistent
+ * split-K tensor-core kernel; above, the tiled tcgen05 tensor-core GEMM, whose order of partial sums follows from the
+ * shape and size_m.  berth_exl3_last_launch names the kernels that ran.  Programmatic-launch contract: up to 32 rows the
+ * kernels start fetching `trellis` while the kernel before them on the stream may still be running, so the weights must
+ * be final before that kernel starts; every other tensor, and above 32 rows the weights too, are touched only after the
+ * predecessor ended. */
 int berth_exl3_linear(const void* a, const void* trellis, void* c, const void* suh, void* a_had,
                       const void* svh, int size_m, int size_k, int size_n, int k_bits,
                       int codebook, int out_fp32, void* stream);
